@@ -457,10 +457,8 @@ enum {
                                   from the eq half tables (0) */
     VG_TUNE_GROUP_SPLIT = 9,   /* round groups: steps with few pairs left spread each pair over three
                                   threads, one per table (1), or keep one thread per pair (0) */
-    VG_TUNE_LAZY_FOLD = 10,    /* sumcheck folds x0 + r (x1 - x0): 0 = canonical difference and the
-                                  three-product (Karatsuba) F_p2 product; 1 = the difference left
-                                  unreduced (x1 + 2p - x0) and a four-product (schoolbook) one,
-                                  fewer integer-ALU steps for more multiply-pipe work */
+    VG_TUNE_LAZY_FOLD = 10,    /* accepted, without effect: the sumcheck folds x0 + r (x1 - x0) have
+                                  one form, the unreduced difference and four products */
     VG_TUNE_GATHER_FUSE = 11,  /* deferred proofs with paired rounds: a phase's table build over
                                   the layer's edges runs inside the pass of its first two rounds
                                   when the table is above the group start (1: the two tables it

@@ -112,8 +112,8 @@ __global__ void __launch_bounds__(128) k_fri_fold_leaf(const fe *__restrict__ c,
     for (int s = 0; s < 65; ++s) {
         const fe *cs = c + (long)s * n;
         fe a0 = cs[k], b0 = cs[k + half], a1 = cs[k + q4], b1 = cs[k + q4 + half];
-        fe y0 = half_fe(vg::fe_fma(a0 + b0, t0, a0 - b0));
-        fe y1 = half_fe(vg::fe_fma(a1 + b1, t1, a1 - b1));
+        fe y0 = half_fe(vg::fe_fma_diff(a0 + b0, t0, b0, a0));
+        fe y1 = half_fe(vg::fe_fma_diff(a1 + b1, t1, b1, a1));
         out[(long)s * nh + k] = y0;
         out[(long)s * nh + k + q4] = y1;
         uint64_t w[8] = {y0.img, y0.real, y1.img, y1.real, h[0], h[1], h[2], h[3]};
@@ -134,7 +134,7 @@ __global__ void k_fri_fold(const fe *__restrict__ c, long n, int t, fe r, const 
         const long s = i / h, k = i - s * h;
         const fe a = c[s * n + k], b = c[s * n + k + h];
         const fe w = r * tw_pow(twi_lo, twi_hi, (uint64_t)k << t);
-        out[i] = half_fe(vg::fe_fma(a + b, w, a - b));
+        out[i] = half_fe(vg::fe_fma_diff(a + b, w, b, a));
     }
 }
 

@@ -179,6 +179,80 @@ __device__ __forceinline__ void block_sum(fe (&v)[K], fe *sm)
     }
 }
 
+// Sums of K values over a grid, exact and fast at the end of a kernel: each
+// 61-bit component is cut into limbs of 21, 21 and 19 bits, one warp-wide
+// integer reduction adds a limb over a warp (26 bits), the warps' sums meet
+// in shared memory (30 bits) and the CTAs' in 64-bit atomics.  A tree of field
+// additions over shuffles (block_sum) is five dependent steps of some 60
+// clocks each at two levels, then again over the CTAs' partials.
+constexpr int LIMBS = 6;   // limbs of a field element
+__device__ __forceinline__ fe fe_from_limbs(unsigned long long i0, unsigned long long i1, unsigned long long i2,
+                                            unsigned long long r0, unsigned long long r1, unsigned long long r2)
+{
+    // limb sums below 2^40: s0 + 2^21 s1 + 2^42 s2 mod p, each term below 2^62
+    fe x;
+    x.img = vg::canon64(i0 + (i1 << 21) + ((i2 << 42) & vg::P) + (i2 >> 19));
+    x.real = vg::canon64(r0 + (r1 << 21) + ((r2 << 42) & vg::P) + (r2 >> 19));
+    return x;
+}
+// limb sums of x over the calling warp (all 32 lanes), the same in every lane
+__device__ __forceinline__ void warp_limbs(fe x, uint32_t (&l)[LIMBS])
+{
+    const uint32_t M = 0x1fffff;
+    l[0] = __reduce_add_sync(0xffffffffu, (uint32_t)x.img & M);
+    l[1] = __reduce_add_sync(0xffffffffu, (uint32_t)(x.img >> 21) & M);
+    l[2] = __reduce_add_sync(0xffffffffu, (uint32_t)(x.img >> 42));
+    l[3] = __reduce_add_sync(0xffffffffu, (uint32_t)x.real & M);
+    l[4] = __reduce_add_sync(0xffffffffu, (uint32_t)(x.real >> 21) & M);
+    l[5] = __reduce_add_sync(0xffffffffu, (uint32_t)(x.real >> 42));
+}
+// Sums acc over the grid (at most 16 warps per CTA, at most 2^10 CTAs): true
+// in the last CTA to finish, with the K totals in tot (shared memory) for
+// every thread; false in the others.  gacc: 6 K words, zero before the launch
+// and again after it, as *counter.
+template <int K>
+__device__ __forceinline__ bool grid_sum(const fe (&acc)[K], uint32_t (&sw)[16][LIMBS * K], fe (&tot)[K],
+                                         unsigned long long *gacc, unsigned *counter)
+{
+    __shared__ bool last;
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        uint32_t l[LIMBS];
+        warp_limbs(acc[k], l);
+        if (lane == 0) {
+#pragma unroll
+            for (int j = 0; j < LIMBS; ++j) sw[wid][LIMBS * k + j] = l[j];
+        }
+    }
+    __syncthreads();
+    unsigned long long s = 0;
+    if (t < LIMBS * K) {
+        for (int w = 0; w < nw; ++w) s += sw[w][t];
+        if (gridDim.x > 1) atomicAdd(&gacc[t], s);
+    }
+    if (gridDim.x > 1) {
+        __threadfence();
+        __syncthreads();
+        if (t == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
+        __syncthreads();
+        if (!last) return false;
+        __threadfence();
+        if (t < LIMBS * K) {
+            s = __ldcg(&gacc[t]);
+            gacc[t] = 0;
+        }
+        if (t == 0) *counter = 0;
+    }
+    // the limbs of value k are in six consecutive threads of the first warps
+    __shared__ unsigned long long sl[LIMBS * K];
+    if (t < LIMBS * K) sl[t] = s;
+    __syncthreads();
+    if (t < K) tot[t] = fe_from_limbs(sl[6 * t], sl[6 * t + 1], sl[6 * t + 2], sl[6 * t + 3], sl[6 * t + 4], sl[6 * t + 5]);
+    __syncthreads();
+    return true;
+}
+
 // sum of `nparts` groups of K partials (layout [part][K]) into out[K]
 int vg_reduce_partials(vg_ctx *ctx, const fe *parts, int nparts, int K, fe *out_dev);
 

@@ -549,8 +549,10 @@ int vg_fft_gkr_launch(vg_fft_gkr *f, int lg, unsigned seed)
     const long prod_blocks = (N + FG_THREADS * PROD_STEPS - 1) / (FG_THREADS * PROD_STEPS);
     f->prod_blocks = prod_blocks;
     const size_t jobs_fe = (jobs.size() * sizeof(HalfJob) + sizeof(fe) - 1) / sizeof(fe);
-    const size_t d_chal = 0, d_jobs = d_chal + n_chal, d_layers = d_jobs + jobs_fe;
-    const size_t d_T = d_layers + (size_t)(lg + 1) * N, d_S = d_T + N / 2 + 1, d_P = d_S + N;
+    // the rounds' tables start on 32-byte boundaries (the paired passes load entries two at a time)
+    auto even = [](size_t x) { return (x + 1) / 2 * 2; };
+    const size_t d_chal = 0, d_jobs = d_chal + n_chal, d_layers = even(d_jobs + jobs_fe);
+    const size_t d_T = d_layers + (size_t)(lg + 1) * N, d_S = even(d_T + N / 2 + 1), d_P = d_S + N;
     const size_t d_half = d_P + NE, d_parts = d_half + half_total, d_end = d_parts + 64 * prod_blocks;
     VG_TRY(vg_ctx_grow_dev(c, (void **)&f->dev, &f->dev_cap, d_end * sizeof(fe)));
     const size_t up_bytes = (n_chal + jobs_fe) * sizeof(fe);

@@ -46,101 +46,136 @@ VG_HD uint64_t subp(uint64_t a, uint64_t b)
 }
 VG_HD uint64_t negp(uint64_t a) { return a ? P - a : 0; }
 
-VG_HD void mul64wide(uint64_t a, uint64_t b, uint64_t &lo, uint64_t &hi)
-{
-#if defined(__CUDA_ARCH__)
-    lo = a * b;
-    hi = __umul64hi(a, b);
-#else
-    unsigned __int128 x = (unsigned __int128)a * b;
-    lo = (uint64_t)x;
-    hi = (uint64_t)(x >> 64);
-#endif
-}
+// 64 x 64 -> 128 bits.  On the device the 128-bit type compiles to four
+// 32 x 32 wide multiplies and three carries; a low and a high product formed
+// separately (a * b, __umul64hi) take seven multiplies, and the multiply pipe
+// (one wide multiply per SM and clock) bounds every field kernel: an F_p2
+// product took 30.1 clocks per warp that way, 26.8 through this type.
+typedef unsigned __int128 u128;
+VG_HD u128 mul128(uint64_t a, uint64_t b) { return (u128)a * b; }
 
 // x mod p for x < 2^64, partly reduced: the result is below 2^61 + 8.
 VG_HD uint64_t foldp(uint64_t x) { return (x & P) + (x >> 61); }
 // x mod p, canonical, for x < 2p: x + 1 reaches 2^61 exactly when x >= p.
 VG_HD uint64_t canonp(uint64_t x) { return (x + ((x + 1) >> 61)) & P; }
 
-// a*b mod p for a, b < 2^61 (canonical).  x = hi*2^64 + lo <= (p-1)^2, and
-// x = (x >> 61) * 2^61 + (x & p) == (x >> 61) + (x & p) (mod p); both terms are
-// at most p and not both p (x < p 2^61 + p), so the sum is below 2p.
-VG_HD uint64_t mulp(uint64_t a, uint64_t b)
+// x mod p as (x & p) + (x >> 61), for x < 2^125: below 2^64.
+VG_HD uint64_t fold128(u128 x)
 {
-    uint64_t lo, hi;
-    mul64wide(a, b, lo, hi);
-    return canonp((lo & P) + ((hi << 3) | (lo >> 61)));
-}
-// a*b mod p, partly reduced (below 2^61 + 8), for a*b < 2^124.
-VG_HD uint64_t mulp_partial(uint64_t a, uint64_t b)
-{
-    uint64_t lo, hi;
-    mul64wide(a, b, lo, hi);
-    return foldp((lo & P) + ((hi << 3) | (lo >> 61)));
-}
-// x = a*b mod p as (x & p) + (x >> 61), not folded further, for a*b < 2^124:
-// below 2^62 when a, b < 2^61 (x >> 61 < 2^61), below 2^61 + 2^63 when
-// a, b < 2^62.
-VG_HD uint64_t mulp_fold1(uint64_t a, uint64_t b)
-{
-    uint64_t lo, hi;
-    mul64wide(a, b, lo, hi);
+    const uint64_t lo = (uint64_t)x, hi = (uint64_t)(x >> 64);
     return (lo & P) + ((hi << 3) | (lo >> 61));
 }
+// z mod p, canonical, for z <= 2^64 - 9.  With z = q 2^61 + s = q p + (q + s),
+// floor(z / p) is q, plus one when q + s >= p, i.e. when q + s + 1 carries into
+// bit 61; so floor(z / p) = (z + q + 1) >> 61 and z minus that many p is
+// (z + floor(z / p)) mod 2^61: seven instructions where a fold and canonp
+// take ten.
+VG_HD uint64_t canon64(uint64_t z)
+{
+    const uint64_t k = (z + (z >> 61) + 1) >> 61;
+    return (z + k) & P;
+}
+
+// a*b mod p for a, b < 2^61 (canonical).  x = a*b <= (p-1)^2, and
+// x = (x >> 61) * 2^61 + (x & p) == (x >> 61) + (x & p) (mod p); both terms are
+// at most p and not both p (x < p 2^61 + p), so the sum is below 2p.
+VG_HD uint64_t mulp(uint64_t a, uint64_t b) { return canonp(fold128(mul128(a, b))); }
 
 // ---- F_{p^2} ----
 VG_HD fe operator+(fe a, fe b) { return fe_make(addp(a.real, b.real), addp(a.img, b.img)); }
 VG_HD fe operator-(fe a, fe b) { return fe_make(subp(a.real, b.real), subp(a.img, b.img)); }
 VG_HD fe operator-(fe a) { return fe_make(negp(a.real), negp(a.img)); }
 
-// (ar + i ai)(br + i bi) = (ar br - ai bi) + i((ar + ai)(br + bi) - ar br - ai bi)
-// For canonical inputs ac = ar br and bd = ai bi are taken once folded
-// (mulp_fold1: below 2^62), t = (ar + ai)(br + bi) (operands below 2^62, the
-// product below 2^124) folded twice (below 2^61 + 5), and the differences as
-// ac + 3p - bd (3p > 2^62 > bd; the sum below 5 2^61) and t + 5p - ac - bd
-// (5p > 2^63 > ac + bd; the sum below 6 2^61), each folded once (below
-// 2^61 + 5) before the final canonical step: the canonical product with two
-// folds fewer than folding every partial product.
-VG_HD fe operator*(fe a, fe b)
+// x + (ar + i ai)(br + i bi) for a, x canonical and b of components at most
+// 2p, with three products whose 128-bit values are combined before any
+// reduction.  With n = 2p - bi and u = ai n (== -ai bi):
+//   real: ar br + u <= 4 p^2;
+//   img:  t - ar br + u = ar bi + ai br + 2p ai <= 6 p^2, t = (ar + ai)(br + bi)
+// (no offset is needed: both are sums of nonnegative products), so each folds
+// once to at most 7p, plus x below 8p = 2^64 - 8, the range of canon64.
+// 26.4 clocks per warp where the products were folded one by one and the
+// result made canonical in two steps (31.9).
+VG_HD fe fe_fma2(fe x, fe a, uint64_t br, uint64_t bi)
 {
-    const uint64_t ac = mulp_fold1(a.real, b.real);
-    const uint64_t bd = mulp_fold1(a.img, b.img);
-    const uint64_t t = foldp(mulp_fold1(a.real + a.img, b.real + b.img));
-    const uint64_t re = foldp(ac + (3 * P - bd));
-    const uint64_t im = foldp(t + (5 * P - ac - bd));
-    return fe_make(canonp(re), canonp(im));
+    const u128 ac = mul128(a.real, br), u = mul128(a.img, 2 * P - bi);
+    const u128 t = mul128(a.real + a.img, br + bi);
+    return fe_make(canon64(fold128(ac + u) + x.real), canon64(fold128(t - ac + u) + x.img));
 }
-
-// x + a*b for canonical x, a, b: x joins the product's two sums before their
-// last fold (ac + 3p - bd + x.real below 6 2^61, t + 5p - ac - bd + x.img
-// below 7 2^61 + 5), so an integer add replaces a canonical one; the same
-// canonical result as x + a * b.
+// x + a*b, all canonical: as fe_fma2 with n = p - bi (p is all ones, so one
+// exclusive or per word), the sums at most 2 p^2 and 3 p^2.
 VG_HD fe fe_fma(fe x, fe a, fe b)
 {
-    const uint64_t ac = mulp_fold1(a.real, b.real);
-    const uint64_t bd = mulp_fold1(a.img, b.img);
-    const uint64_t t = foldp(mulp_fold1(a.real + a.img, b.real + b.img));
-    const uint64_t re = foldp(ac + (3 * P - bd) + x.real);
-    const uint64_t im = foldp(t + (5 * P - ac - bd) + x.img);
-    return fe_make(canonp(re), canonp(im));
+    const u128 ac = mul128(a.real, b.real), u = mul128(a.img, b.img ^ P);
+    const u128 t = mul128(a.real + a.img, b.real + b.img);
+    return fe_make(canon64(fold128(ac + u) + x.real), canon64(fold128(t - ac + u) + x.img));
+}
+VG_HD fe operator*(fe a, fe b)
+{
+    const u128 ac = mul128(a.real, b.real), u = mul128(a.img, b.img ^ P);
+    const u128 t = mul128(a.real + a.img, b.real + b.img);
+    return fe_make(canon64(fold128(ac + u)), canon64(fold128(t - ac + u)));
+}
+// x + m (v1 - v0), all canonical, the difference left unreduced (v1 + p - v0)
+VG_HD fe fe_fma_diff(fe x, fe m, fe v0, fe v1)
+{
+    return fe_fma2(x, m, v1.real + P - v0.real, v1.img + P - v0.img);
+}
+// a*b + c*d, all canonical: the products meet in 128 bits (the real sum at
+// most 4 p^2, the imaginary one 6 p^2) and are reduced once, 36.6 clocks per
+// warp where a product and a fused one took 50.7.
+VG_HD fe fe_dot2(fe a, fe b, fe c, fe d)
+{
+    const u128 ac = mul128(a.real, b.real) + mul128(c.real, d.real);
+    const u128 u = mul128(a.img, b.img ^ P) + mul128(c.img, d.img ^ P);
+    const u128 t = mul128(a.real + a.img, b.real + b.img) + mul128(c.real + c.img, d.real + d.img);
+    return fe_make(canon64(fold128(ac + u)), canon64(fold128(t - ac + u)));
+}
+
+// The fold x0 + r (x1 - x0) by a challenge used many times.  The constants are
+// 8 rr, 8 ri and 8 (p - ri): the factor 8 puts floor(y / 2^61) of a sum of
+// products y into the high word of 8 y, and y mod 2^61 is its low word >> 3, so
+// the reduction needs no shift across words.  Four products (the imaginary
+// part as dr ri + di rr) with the differences unreduced (x1 + p - x0 < 2p):
+// 8 y < 2 (2p)(8p) < 2^127, high word < 4p, low >> 3 <= p, plus x0: below 6p.
+// 30 clocks per warp in the paired rounds where a canonical difference and
+// fe_fma took 38.
+struct fold_r {
+    uint64_t r, i, n;
+};
+VG_HD fold_r fold_prep(fe r)
+{
+    fold_r f;
+    f.r = r.real << 3;
+    f.i = r.img << 3;
+    f.n = (r.img ^ P) << 3;
+    return f;
+}
+VG_HD uint64_t fold128_8(u128 x) { return (uint64_t)(x >> 64) + ((uint64_t)x >> 3); }
+VG_HD fe fe_fold(fe x0, fe x1, fold_r f)
+{
+    const uint64_t dr = x1.real + P - x0.real, di = x1.img + P - x0.img;
+    return fe_make(canon64(fold128_8(mul128(dr, f.r) + mul128(di, f.n)) + x0.real),
+                   canon64(fold128_8(mul128(dr, f.i) + mul128(di, f.r)) + x0.img));
 }
 
 VG_HD fe fe_double(fe a) { return a + a; }
 
-// x0 + r (x1 - x0) for canonical x0, x1, r with the difference left
-// unreduced: x1 + 2p - x0 < 3p < 2^63 per component, multiplied by r with
-// four partial products (no sums of operands), each below 3p * p < 2^124,
-// mulp_partial's range.  Fewer integer-ALU steps than the canonical
-// subtraction and three-product form; the same canonical result.
-VG_HD fe fold_lazy(fe x0, fe x1, fe r)
+// Operands in F_p (imaginary part zero), such as every layer value of a
+// circuit (integer inputs, gates with coefficients in F_p): two products of
+// the field's three or four.  v is at most 2p, so each part is below 2p^2.
+VG_HD fe fe_fma_real(fe x, fe m, uint64_t v)
 {
-    const uint64_t dr = x1.real + 2 * P - x0.real, di = x1.img + 2 * P - x0.img;
-    const uint64_t ac = mulp_partial(dr, r.real), bd = mulp_partial(di, r.img);
-    const uint64_t ad = mulp_partial(dr, r.img), bc = mulp_partial(di, r.real);
-    const uint64_t re = foldp(ac + (4 * P - bd));
-    const uint64_t im = foldp(ad + bc);
-    return x0 + fe_make(canonp(re), canonp(im));
+    return fe_make(canon64(fold128(mul128(m.real, v)) + x.real), canon64(fold128(mul128(m.img, v)) + x.img));
+}
+VG_HD fe fe_mul_real(fe m, uint64_t v)
+{
+    return fe_make(canon64(fold128(mul128(m.real, v))), canon64(fold128(mul128(m.img, v))));
+}
+// x0 + r (x1 - x0) for x0, x1 in F_p (canonical)
+VG_HD fe fe_fold_real(uint64_t x0, uint64_t x1, fold_r f)
+{
+    const uint64_t d = x1 + P - x0;
+    return fe_make(canon64(fold128_8(mul128(d, f.r)) + x0), canon64(fold128_8(mul128(d, f.i))));
 }
 
 // a * 2^k for canonical a and 0 <= k <= 60: since 2^61 = 1 (mod p), this is a

@@ -82,41 +82,48 @@ __global__ void k_eval_input(const int64_t *__restrict__ u, long n, fe *__restri
     if (g < n) out[g] = from_int32((int32_t)u[g]);
 }
 
-// zk_prover::evaluate, one layer (zk_prover.cpp:68-150)
+// zk_prover::evaluate, one layer (zk_prover.cpp:68-150).  The input values
+// are integers and no gate leaves F_p, so every layer value has a zero
+// imaginary part: the kernel reads and computes real parts only (one product
+// per gate in place of an F_p2 product) and writes {0, value}.
+__device__ __forceinline__ uint64_t eval_gate(int t, uint32_t u, uint32_t v, const fe *__restrict__ prev)
+{
+    switch (t) {
+    case 0: return vg::addp(prev[u].real, prev[v].real);
+    case 1: return vg::mulp(prev[u].real, prev[v].real);
+    case 3: return from_int32((int32_t)u).real;
+    case 4:
+    case 10: return prev[u].real;
+    case 5: {
+        uint64_t r = 0;
+        for (uint32_t k = u; k < v; ++k) r = vg::addp(r, prev[k].real);
+        return r;
+    }
+    case 6: return vg::subp(1, prev[u].real);
+    case 7: return vg::subp(prev[u].real, prev[v].real);
+    case 8: {
+        const uint64_t x = prev[u].real, y = prev[v].real, xy = vg::mulp(x, y);
+        return vg::subp(vg::addp(x, y), vg::addp(xy, xy));
+    }
+    case 9: {
+        const uint64_t x = prev[u].real, y = prev[v].real;
+        return vg::subp(y, vg::mulp(x, y));
+    }
+    case 12: {   // sum_k prev[k] 2^(k-u), Horner from the top
+        uint64_t r = 0;
+        for (long k = (long)v; k >= (long)u; --k) r = vg::addp(vg::addp(r, r), prev[k].real);
+        return r;
+    }
+    case 13: return vg::mulp(prev[u].real, vg::subp(1, prev[v].real));
+    default: return 0;   // 2 (dummy) and unknown types evaluate to 0
+    }
+}
 __global__ void k_eval_layer(const uint8_t *__restrict__ ty, const uint32_t *__restrict__ uu,
                              const uint32_t *__restrict__ vv, long n, const fe *__restrict__ prev,
                              fe *__restrict__ out)
 {
-    for (long g = blockIdx.x * (long)blockDim.x + threadIdx.x; g < n; g += (long)gridDim.x * blockDim.x) {
-        const uint32_t u = uu[g], v = vv[g];
-        fe r = vg::fe_zero();
-        switch (ty[g]) {
-        case 0: r = prev[u] + prev[v]; break;
-        case 1: r = prev[u] * prev[v]; break;
-        case 3: r = from_int32((int32_t)u); break;
-        case 4:
-        case 10: r = prev[u]; break;
-        case 5:
-            for (uint32_t k = u; k < v; ++k) r = r + prev[k];
-            break;
-        case 6: r = vg::fe_one() - prev[u]; break;
-        case 7: r = prev[u] - prev[v]; break;
-        case 8: {
-            fe x = prev[u], y = prev[v], xy = x * y;
-            r = (x + y) - (xy + xy);
-        } break;
-        case 9: {
-            fe x = prev[u], y = prev[v];
-            r = y - x * y;
-        } break;
-        case 12:   // sum_k prev[k] 2^(k-u), Horner from the top
-            for (long k = (long)v; k >= (long)u; --k) r = (r + r) + prev[k];
-            break;
-        case 13: r = prev[u] * (vg::fe_one() - prev[v]); break;
-        default: break;   // 2 (dummy) and unknown types evaluate to 0
-        }
-        out[g] = r;
-    }
+    for (long g = blockIdx.x * (long)blockDim.x + threadIdx.x; g < n; g += (long)gridDim.x * blockDim.x)
+        out[g] = vg::fe_make(eval_gate(ty[g], uu[g], vv[g], prev), 0);
 }
 
 // ------------------------------------------------------------ eq tables
@@ -186,7 +193,7 @@ struct BetaG {
     __device__ __forceinline__ fe at(long i) const
     {
         if (tab) return tab[i];
-        return vg::fe_fma(f0[i & mask] * s0[i >> fh], f1[i & mask], s1[i >> fh]);
+        return vg::fe_dot2(f0[i & mask], s0[i >> fh], f1[i & mask], s1[i >> fh]);
     }
 };
 struct BetaU {
@@ -424,7 +431,8 @@ __global__ void k_medium_keys(const uint32_t *__restrict__ off, long N, uint32_t
     }
 }
 
-// contribution of one edge to the phase-1 tables (k_phase1_scatter's cases)
+// contribution of one edge to the phase-1 tables (k_phase1_scatter's cases);
+// the other operand is a layer value, in F_p
 __device__ __forceinline__ void edge1(int tk, uint32_t gv, uint32_t o, const BetaG &bg, const fe *__restrict__ prev, fe &am,
                                       fe &av)
 {
@@ -432,22 +440,22 @@ __device__ __forceinline__ void edge1(int tk, uint32_t gv, uint32_t o, const Bet
     const fe b = bg.at(gv);
     if (bg.save) bg.save[gv] = b;   // every edge of a gate stores the same value
     switch (t) {
-    case 0: av = vg::fe_fma(av, prev[o], b); am = am + b; break;
-    case 1: am = vg::fe_fma(am, prev[o], b); break;
+    case 0: av = vg::fe_fma_real(av, b, prev[o].real); am = am + b; break;
+    case 1: am = vg::fe_fma_real(am, b, prev[o].real); break;
     case 4:
     case 5:
     case 10: am = am + b; break;
     case 12: am = am + vg::fe_mul_pow2(b, tk >> 8); break;
     case 6: am = am - b; av = av + b; break;
-    case 7: av = av - prev[o] * b; am = am + b; break;
+    case 7: av = vg::fe_fma_real(av, b, prev[o].real ^ vg::P); am = am + b; break;   // - b prev
     case 8: {
-        const fe x = b * prev[o];
+        const fe x = vg::fe_mul_real(b, prev[o].real);
         av = av + x;
         am = am + (b - (x + x));
     } break;
-    case 13: am = am + (b - b * prev[o]); break;
+    case 13: am = am + (b - vg::fe_mul_real(b, prev[o].real)); break;
     case 9: {
-        const fe x = b * prev[o];
+        const fe x = vg::fe_mul_real(b, prev[o].real);
         av = av + x;
         am = am - x;
     } break;
@@ -642,33 +650,21 @@ struct RoundGroup {
     const fe *r;        // fold challenge of each round (device memory, nsteps values)
 };
 
-// x0 + r (x1 - x0); LAZY: the unreduced difference and the four-product
-// form (vg::fold_lazy), the same canonical value
-template <bool LAZY>
-__device__ __forceinline__ fe rg_fold(fe x0, fe x1, fe r)
-{
-    if (LAZY) return vg::fold_lazy(x0, x1, r);
-    return vg::fe_fma(x0, r, x1 - x0);
-}
-
 // A round's sums over one pair: (m0 + ma x)(v0 + va x) + a0 + aa x has x^2
-// term ma va, x term ma v0 + m0 va + aa = m1 v1 - m0 v0 - ma va + aa (three
-// products, not four) and constant m0 v0 + a0.  FULL = false leaves out the
-// x term (the group's epilogue forms it from the round's claim): two products.
+// term ma va, value m0 v0 + a0 at 0 and m1 v1 + a1 at 1, and its x term is
+// the value at 1 minus the other two.  acc[0] and acc[2] collect the x^2 terms
+// and the values at 0; with FULL acc[1] collects the values at 1 (three
+// products; rg_sums_end turns it into the x term), without it the x term is
+// left out (the group's epilogue forms it from the round's claim): two
+// products, each added inside its last fold.
 template <bool FULL = true>
 __device__ __forceinline__ void rg_sums(fe v0, fe v1, fe a0, fe a1, fe m0, fe m1, fe (&acc)[3])
 {
-    const fe va = v1 - v0, ma = m1 - m0;
-    if (FULL) {
-        const fe p2 = ma * va, p0 = m0 * v0;
-        acc[0] = acc[0] + p2;
-        acc[1] = acc[1] + ((m1 * v1 - p0 - p2) + (a1 - a0));
-        acc[2] = acc[2] + p0 + a0;
-    } else {   // each product added inside its last fold (vg::fe_fma)
-        acc[0] = vg::fe_fma(acc[0], ma, va);
-        acc[2] = vg::fe_fma(acc[2] + a0, m0, v0);
-    }
+    acc[0] = vg::fe_fma_diff(acc[0], m1 - m0, v0, v1);
+    acc[2] = vg::fe_fma(acc[2] + a0, m0, v0);
+    if (FULL) acc[1] = vg::fe_fma(acc[1] + a1, m1, v1);
 }
+__device__ __forceinline__ void rg_sums_end(fe (&acc)[3]) { acc[1] = (acc[1] - acc[2]) - acc[0]; }
 
 // The x term of a round that follows another round of its phase, from the
 // others: the round's polynomial s(x) = a x^2 + b x + c sums to the claim
@@ -751,7 +747,7 @@ __device__ __forceinline__ void rg_derive_smem(fe *tot, const fe *sr, fe *d, int
 // after the fence and counter that order every CTA's writes before it.
 // SPLIT: the three-thread steps (VG_TUNE_GROUP_SPLIT) are compiled in only
 // when asked for, for the same reason
-template <bool LAZY, bool SPLIT>
+template <bool SPLIT>
 __global__ void __launch_bounds__(RG_THREADS) k_round_group(const fe *__restrict__ xV, const fe *__restrict__ xA,
                                                             const fe *__restrict__ xM, long n_in, RoundGroup G,
                                                             fe *yV, fe *yA, fe *yM, fe *__restrict__ parts,
@@ -838,7 +834,7 @@ __global__ void __launch_bounds__(RG_THREADS) k_round_group(const fe *__restrict
         // first step: from global into shared
         {
             fe acc[3] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
-            const fe r = sr[st0];
+            const vg::fold_r r = vg::fold_prep(sr[st0]);
             for (long k = t; k < m / 2; k += RG_THREADS) {
                 fe v0, v1, a0, a1, m0v, m1v;
                 if (nofold) {
@@ -848,12 +844,12 @@ __global__ void __launch_bounds__(RG_THREADS) k_round_group(const fe *__restrict
                     m0v = ld_fe_cg(X2 + b); m1v = ld_fe_cg(X2 + b + 1);
                 } else {
                     const long b = base + 4 * k;
-                    v0 = rg_fold<LAZY>(ld_fe_cg(X0 + b), ld_fe_cg(X0 + b + 1), r);
-                    v1 = rg_fold<LAZY>(ld_fe_cg(X0 + b + 2), ld_fe_cg(X0 + b + 3), r);
-                    a0 = rg_fold<LAZY>(ld_fe_cg(X1 + b), ld_fe_cg(X1 + b + 1), r);
-                    a1 = rg_fold<LAZY>(ld_fe_cg(X1 + b + 2), ld_fe_cg(X1 + b + 3), r);
-                    m0v = rg_fold<LAZY>(ld_fe_cg(X2 + b), ld_fe_cg(X2 + b + 1), r);
-                    m1v = rg_fold<LAZY>(ld_fe_cg(X2 + b + 2), ld_fe_cg(X2 + b + 3), r);
+                    v0 = vg::fe_fold(ld_fe_cg(X0 + b), ld_fe_cg(X0 + b + 1), r);
+                    v1 = vg::fe_fold(ld_fe_cg(X0 + b + 2), ld_fe_cg(X0 + b + 3), r);
+                    a0 = vg::fe_fold(ld_fe_cg(X1 + b), ld_fe_cg(X1 + b + 1), r);
+                    a1 = vg::fe_fold(ld_fe_cg(X1 + b + 2), ld_fe_cg(X1 + b + 3), r);
+                    m0v = vg::fe_fold(ld_fe_cg(X2 + b), ld_fe_cg(X2 + b + 1), r);
+                    m1v = vg::fe_fold(ld_fe_cg(X2 + b + 2), ld_fe_cg(X2 + b + 3), r);
                 }
                 const int i0 = rg_ix(2 * k), i1 = rg_ix(2 * k + 1);
                 sV[i0] = v0; sV[i1] = v1;
@@ -861,11 +857,12 @@ __global__ void __launch_bounds__(RG_THREADS) k_round_group(const fe *__restrict
                 sM[i0] = m0v; sM[i1] = m1v;
                 rg_sums(v0, v1, a0, a1, m0v, m1v, acc);
             }
+            rg_sums_end(acc);
             rg_warp_add(acc, wsum, st0, m / 2);
         }
         // further steps in shared memory: fold m -> m/2, sums over m/4 pairs
         for (int st = st0 + 1; st < st1; ++st) {
-            const fe r = sr[st];
+            const vg::fold_r r = vg::fold_prep(sr[st]);
             const long npairs = m / 4;
             if (SPLIT && 3 * npairs <= RG_THREADS) {
                 // few pairs: three threads per pair, one per table, each
@@ -879,8 +876,8 @@ __global__ void __launch_bounds__(RG_THREADS) k_round_group(const fe *__restrict
                 fe f0 = vg::fe_zero(), f1 = vg::fe_zero();
                 __syncthreads();
                 if (act) {
-                    f0 = rg_fold<LAZY>(tab[rg_ix(4 * pp)], tab[rg_ix(4 * pp + 1)], r);
-                    f1 = rg_fold<LAZY>(tab[rg_ix(4 * pp + 2)], tab[rg_ix(4 * pp + 3)], r);
+                    f0 = vg::fe_fold(tab[rg_ix(4 * pp)], tab[rg_ix(4 * pp + 1)], r);
+                    f1 = vg::fe_fold(tab[rg_ix(4 * pp + 2)], tab[rg_ix(4 * pp + 3)], r);
                     stage[6 * pp + 2 * role] = f0;
                     stage[6 * pp + 2 * role + 1] = f1;
                 }
@@ -903,9 +900,9 @@ __global__ void __launch_bounds__(RG_THREADS) k_round_group(const fe *__restrict
             const bool act = t < npairs;   // m / 4 <= RG_CHUNK / 4 = RG_THREADS: at most one pair per thread
             if (act) {
                 const int b0 = rg_ix(4 * t), b1 = rg_ix(4 * t + 1), b2 = rg_ix(4 * t + 2), b3 = rg_ix(4 * t + 3);
-                v0 = rg_fold<LAZY>(sV[b0], sV[b1], r); v1 = rg_fold<LAZY>(sV[b2], sV[b3], r);
-                a0 = rg_fold<LAZY>(sA[b0], sA[b1], r); a1 = rg_fold<LAZY>(sA[b2], sA[b3], r);
-                m0v = rg_fold<LAZY>(sM[b0], sM[b1], r); m1v = rg_fold<LAZY>(sM[b2], sM[b3], r);
+                v0 = vg::fe_fold(sV[b0], sV[b1], r); v1 = vg::fe_fold(sV[b2], sV[b3], r);
+                a0 = vg::fe_fold(sA[b0], sA[b1], r); a1 = vg::fe_fold(sA[b2], sA[b3], r);
+                m0v = vg::fe_fold(sM[b0], sM[b1], r); m1v = vg::fe_fold(sM[b2], sM[b3], r);
                 rg_sums<false>(v0, v1, a0, a1, m0v, m1v, acc);
             }
             __syncthreads();
@@ -1009,42 +1006,35 @@ __global__ void k_vu(const fe *__restrict__ last6, fe r, fe addend, fe *__restri
 }
 
 // ------------------------------------------------------------ round kernel
-template <bool LAZY>
-__device__ __forceinline__ fe fold(fe x0, fe x1, fe r)
-{
-    if (LAZY) return vg::fold_lazy(x0, x1, r);
-    return vg::fe_fma(x0, r, x1 - x0);
-}
-
-// The block partials are reduced by the last block to finish (a counter in
-// device memory decides which one), so one launch returns the round sums.
+// The sums are reduced over the grid by grid_sum, so one launch returns them.
 // The fold challenge comes from device memory (rp), so a captured launch
 // sequence can be replayed with the next proof's challenges.
 // A folding round's x term follows from the claim (rg_derive): prev3 holds
 // the previous round's sums (the record before it, or on a synchronous
 // object the sums buffer out3 itself, read before it is written).
-template <bool FOLD, int THREADS, bool LAZY>
+template <bool FOLD, int THREADS>
 __global__ void __launch_bounds__(THREADS) k_round(const fe *__restrict__ xV, const fe *__restrict__ xAV,
                                                        const fe *__restrict__ xAM, long npairs,
                                                        const fe *__restrict__ rp,
                                                        fe *__restrict__ yV, fe *__restrict__ yAV, fe *__restrict__ yAM,
-                                                       fe *__restrict__ parts, unsigned *__restrict__ counter,
+                                                       unsigned long long *__restrict__ gacc, unsigned *__restrict__ counter,
                                                        fe *out3, fe *__restrict__ last6, const fe *prev3)
 {
-    __shared__ fe sm[3 * 32];
-    __shared__ bool last;
+    __shared__ uint32_t sw[16][LIMBS * 3];
+    __shared__ fe tot[3];
     const fe r = FOLD ? *rp : vg::fe_zero();
+    const vg::fold_r fr = vg::fold_prep(r);
     fe acc[3] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < npairs; i += (long)gridDim.x * blockDim.x) {
         fe v0, v1, a0, a1, m0, m1;
         if (FOLD) {
             const long b = 4 * i;
-            v0 = fold<LAZY>(xV[b], xV[b + 1], r);
-            v1 = fold<LAZY>(xV[b + 2], xV[b + 3], r);
-            a0 = fold<LAZY>(xAV[b], xAV[b + 1], r);
-            a1 = fold<LAZY>(xAV[b + 2], xAV[b + 3], r);
-            m0 = fold<LAZY>(xAM[b], xAM[b + 1], r);
-            m1 = fold<LAZY>(xAM[b + 2], xAM[b + 3], r);
+            v0 = vg::fe_fold(xV[b], xV[b + 1], fr);
+            v1 = vg::fe_fold(xV[b + 2], xV[b + 3], fr);
+            a0 = vg::fe_fold(xAV[b], xAV[b + 1], fr);
+            a1 = vg::fe_fold(xAV[b + 2], xAV[b + 3], fr);
+            m0 = vg::fe_fold(xAM[b], xAM[b + 1], fr);
+            m1 = vg::fe_fold(xAM[b + 2], xAM[b + 3], fr);
             yV[2 * i] = v0; yV[2 * i + 1] = v1;
             yAV[2 * i] = a0; yAV[2 * i + 1] = a1;
             yAM[2 * i] = m0; yAM[2 * i + 1] = m1;
@@ -1058,75 +1048,34 @@ __global__ void __launch_bounds__(THREADS) k_round(const fe *__restrict__ xV, co
         }
         rg_sums<!FOLD>(v0, v1, a0, a1, m0, m1, acc);
     }
-    block_sum<3>(acc, sm);
+    if (!FOLD) rg_sums_end(acc);
+    if (!grid_sum<3>(acc, sw, tot, gacc, counter)) return;
     if (threadIdx.x == 0) {
-        parts[3 * blockIdx.x + 0] = acc[0];
-        parts[3 * blockIdx.x + 1] = acc[1];
-        parts[3 * blockIdx.x + 2] = acc[2];
-        __threadfence();
-        last = atomicAdd(counter, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    fe tot[3] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            fe x;
-            x.img = __ldcg(&parts[3 * b + k].img);
-            x.real = __ldcg(&parts[3 * b + k].real);
-            tot[k] = tot[k] + x;
-        }
-    }
-    __syncthreads();
-    block_sum<3>(tot, sm);
-    if (threadIdx.x == 0) {
+        fe x[3] = {tot[0], tot[1], tot[2]};
         if (FOLD) {
             fe prev[3];
             ld_rec3(prev, prev3);
-            rg_derive(tot, prev, r);
+            rg_derive(x, prev, r);
         }
-        out3[0] = tot[0];
-        out3[1] = tot[1];
-        out3[2] = tot[2];
-        *counter = 0;
+        out3[0] = x[0];
+        out3[1] = x[1];
+        out3[2] = x[2];
     }
 }
 
-// The two rounds' sums of a paired pass: one block reduction of the six
-// values, a CTA's partials into parts, and the last CTA to finish (a counter
-// in device memory decides which) adds every CTA's into the two records.
+// The two rounds' sums of a paired pass, six values in one grid_sum; the
+// last CTA to finish writes the two records.
 // The second round's x term, and the first's when it folds (derive_a), follow
 // from the claims (rg_derive): the first round's claim is the record before
 // out_a at ra, the second's the first round's polynomial at rb.
-__device__ __forceinline__ void round2_finish(const fe (&sa)[3], const fe (&sb)[3], fe *sm, bool &last,
-                                              fe *__restrict__ parts, unsigned *__restrict__ counter,
-                                              fe *out_a, fe *__restrict__ out_b, bool derive_a, fe ra, fe rb)
+__device__ __forceinline__ void round2_finish(const fe (&sa)[3], const fe (&sb)[3], unsigned long long *__restrict__ gacc,
+                                              unsigned *__restrict__ counter, fe *out_a, fe *__restrict__ out_b,
+                                              bool derive_a, fe ra, fe rb)
 {
-    fe acc[6] = {sa[0], sa[1], sa[2], sb[0], sb[1], sb[2]};
-    block_sum<6>(acc, sm);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < 6; ++k) parts[6 * blockIdx.x + k] = acc[k];
-        __threadfence();
-        last = atomicAdd(counter, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    fe tot[6] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero(), vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            fe x;
-            x.img = __ldcg(&parts[6 * b + k].img);
-            x.real = __ldcg(&parts[6 * b + k].real);
-            tot[k] = tot[k] + x;
-        }
-    }
-    __syncthreads();
-    block_sum<6>(tot, sm);
+    __shared__ uint32_t sw[16][LIMBS * 6];
+    __shared__ fe tot[6];
+    const fe acc[6] = {sa[0], sa[1], sa[2], sb[0], sb[1], sb[2]};
+    if (!grid_sum<6>(acc, sw, tot, gacc, counter)) return;
     if (threadIdx.x == 0) {
         fe A[3] = {tot[0], tot[1], tot[2]}, B[3] = {tot[3], tot[4], tot[5]};
         if (derive_a) {
@@ -1137,73 +1086,145 @@ __device__ __forceinline__ void round2_finish(const fe (&sa)[3], const fe (&sb)[
         rg_derive(B, A, rb);
         out_a[0] = A[0]; out_a[1] = A[1]; out_a[2] = A[2];
         out_b[0] = B[0]; out_b[1] = B[1]; out_b[2] = B[2];
-        *counter = 0;
     }
+}
+
+// Entries 2k, 2k + 1 of a table in one 32-byte load (p 32-byte aligned)
+__device__ __forceinline__ void ld_pair(const fe *p, fe &x0, fe &x1)
+{
+    asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];"
+        : "=l"(x0.img), "=l"(x0.real), "=l"(x1.img), "=l"(x1.real)
+        : "l"(p));
+}
+__device__ __forceinline__ fe sel_fe(bool c, fe a, fe b) { return c ? a : b; }
+__device__ __forceinline__ fe shfl_xor_fe(fe x, int mask)
+{
+    fe r;
+    r.real = __shfl_xor_sync(0xffffffffu, x.real, mask);
+    r.img = __shfl_xor_sync(0xffffffffu, x.img, mask);
+    return r;
+}
+// Two rows of 32 values, x and y, whose neighbours (lanes l and l ^ bit) form
+// pairs: lanes with the bit clear take row x's pairs, the others row y's.
+// own: this lane's value of its pair, other: the neighbour's.
+__device__ __forceinline__ void pair_up(fe x, fe y, bool hi, int bit, fe &own, fe &other)
+{
+    own = sel_fe(hi, y, x);
+    other = shfl_xor_fe(sel_fe(hi, x, y), bit);
+}
+
+// The sums of one pair held as own / other (hi: own is the odd entry); the
+// x^2 term does not depend on the order
+__device__ __forceinline__ void pair_sums(fe vo, fe vx, fe ao, fe ax, fe mo, fe mx, bool hi, fe (&acc)[3])
+{
+    acc[0] = vg::fe_fma_diff(acc[0], mx - mo, vo, vx);
+    acc[2] = vg::fe_fma(acc[2] + sel_fe(hi, ax, ao), sel_fe(hi, mx, mo), sel_fe(hi, vx, vo));
 }
 
 // Two consecutive rounds in one pass over tables above the group start
 // (deferred mode): rounds only combine neighbouring entries and both
-// challenges are known, so a thread takes 8 consecutive entries of each table
-// (4 when the first round is the unfolded one after a phase init), folds them
-// with ra into 4, adds the first round's sums over those two pairs, folds
-// with rb into 2, adds the second round's sums over that pair and writes the
-// 2 entries: one read of the tables for two rounds, a quarter of them
-// written.  Both rounds' sums go through one block reduction and the
-// last-block pass (6 values per CTA).
-// (both challenges from device memory: rp[0] for the first fold, rp[1] for
-// the second)
-template <bool FOLD, int THREADS, bool LAZY>
-__global__ void __launch_bounds__(THREADS) k_round2(const fe *__restrict__ xV, const fe *__restrict__ xAV,
+// challenges are known.  A warp takes 256 consecutive entries of each table
+// (128 when the first round is the unfolded one after a phase init), folds them
+// with ra, adds the first round's sums over the folded pairs, folds with rb,
+// adds the second round's sums and writes a quarter of what it read: one read
+// of the tables for two rounds.  A lane loads pairs (32 bytes, the rows of a
+// warp contiguous) and the second level's pairs meet by exchanging one value
+// with the neighbour lane, so every load and store is contiguous over the
+// warp; a thread that took 8 consecutive entries touched 32 lines with every
+// load and the pass ran at a quarter of its arithmetic's rate (157 us on
+// 2^22-entry tables).  Both rounds' sums go through one block reduction and
+// the last-block pass (6 values per CTA); the grid is what is resident at
+// once, looping.  (both challenges from device memory: rp[0] for the first
+// fold, rp[1] for the second)
+template <bool FOLD, int THREADS>
+__global__ void __launch_bounds__(THREADS, 512 / THREADS) k_round2(const fe *__restrict__ xV, const fe *__restrict__ xAV,
                                                     const fe *__restrict__ xAM, long nquads,
                                                     const fe *__restrict__ rp,
                                                     fe *__restrict__ yV, fe *__restrict__ yAV, fe *__restrict__ yAM,
-                                                    fe *__restrict__ parts, unsigned *__restrict__ counter,
+                                                    unsigned long long *__restrict__ gacc, unsigned *__restrict__ counter,
                                                     fe *__restrict__ out_a, fe *__restrict__ out_b)
 {
-    __shared__ fe sm[6 * 32];
-    __shared__ bool last;
     const fe ra = FOLD ? rp[0] : vg::fe_zero(), rb = rp[1];
+    const int lane = threadIdx.x & 31;
+    const bool hi = lane & 1, hi2 = lane & 2;
+    const long nwarps = (long)gridDim.x * (THREADS / 32), w0 = (blockIdx.x * (long)THREADS + threadIdx.x) >> 5;
     fe sa[3] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero()}, sb[3] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nquads; i += (long)gridDim.x * blockDim.x) {
-        fe v[4], a[4], m[4];
-        if (FOLD) {
-            const long b = 8 * i;
+    if (FOLD) {
+        // own + r (other - own) is the fold for the even entry's lane; the odd
+        // entry's lane folds with 1 - r
+        const vg::fold_r fa = vg::fold_prep(ra), fb = vg::fold_prep(hi ? vg::fe_one() - rb : rb);
+        for (long w = w0; w < (nquads >> 5); w += nwarps) {
+            fe v[4], a[4], m[4];
+            const long b = 256 * w + 2 * lane;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                v[k] = fold<LAZY>(xV[b + 2 * k], xV[b + 2 * k + 1], ra);
-                a[k] = fold<LAZY>(xAV[b + 2 * k], xAV[b + 2 * k + 1], ra);
-                m[k] = fold<LAZY>(xAM[b + 2 * k], xAM[b + 2 * k + 1], ra);
+                fe x0, x1;
+                ld_pair(xV + b + 64 * k, x0, x1);
+                v[k] = vg::fe_fold(x0, x1, fa);
+                ld_pair(xAM + b + 64 * k, x0, x1);
+                m[k] = vg::fe_fold(x0, x1, fa);
+                ld_pair(xAV + b + 64 * k, x0, x1);
+                a[k] = vg::fe_fold(x0, x1, fa);
             }
-        } else {
-            const long b = 4 * i;
+            fe fv[2], fa2[2], fm[2];
+            const long o = 64 * w + (hi ? 16 : 0) + (lane >> 1);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                v[k] = xV[b + k];
-                a[k] = xAV[b + k];
-                m[k] = xAM[b + k];
+            for (int h = 0; h < 2; ++h) {
+                fe vo, vx, ao, ax, mo, mx;
+                pair_up(v[2 * h], v[2 * h + 1], hi, 1, vo, vx);
+                pair_up(m[2 * h], m[2 * h + 1], hi, 1, mo, mx);
+                pair_up(a[2 * h], a[2 * h + 1], hi, 1, ao, ax);
+                pair_sums(vo, vx, ao, ax, mo, mx, hi, sa);
+                fv[h] = vg::fe_fold(vo, vx, fb);
+                fm[h] = vg::fe_fold(mo, mx, fb);
+                fa2[h] = vg::fe_fold(ao, ax, fb);
+                yV[o + 32 * h] = fv[h];
+                yAM[o + 32 * h] = fm[h];
+                yAV[o + 32 * h] = fa2[h];
             }
+            // the outputs' neighbours are two lanes apart
+            fe vo, vx, ao, ax, mo, mx;
+            pair_up(fv[0], fv[1], hi2, 2, vo, vx);
+            pair_up(fm[0], fm[1], hi2, 2, mo, mx);
+            pair_up(fa2[0], fa2[1], hi2, 2, ao, ax);
+            pair_sums(vo, vx, ao, ax, mo, mx, hi2, sb);
         }
-        rg_sums<!FOLD>(v[0], v[1], a[0], a[1], m[0], m[1], sa);
-        rg_sums<!FOLD>(v[2], v[3], a[2], a[3], m[2], m[3], sa);
-        const fe v0 = fold<LAZY>(v[0], v[1], rb), v1 = fold<LAZY>(v[2], v[3], rb);
-        const fe a0 = fold<LAZY>(a[0], a[1], rb), a1 = fold<LAZY>(a[2], a[3], rb);
-        const fe m0 = fold<LAZY>(m[0], m[1], rb), m1 = fold<LAZY>(m[2], m[3], rb);
-        rg_sums<false>(v0, v1, a0, a1, m0, m1, sb);
-        yV[2 * i] = v0; yV[2 * i + 1] = v1;
-        yAV[2 * i] = a0; yAV[2 * i + 1] = a1;
-        yAM[2 * i] = m0; yAM[2 * i + 1] = m1;
+    } else {
+        const vg::fold_r fb = vg::fold_prep(rb);
+        for (long w = w0; w < (nquads >> 5); w += nwarps) {
+            fe v[2], a[2], m[2];
+            const long b = 128 * w + 2 * lane;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                fe v0, v1, a0, a1, m0, m1;
+                ld_pair(xV + b + 64 * k, v0, v1);
+                ld_pair(xAM + b + 64 * k, m0, m1);
+                ld_pair(xAV + b + 64 * k, a0, a1);
+                rg_sums(v0, v1, a0, a1, m0, m1, sa);
+                const long o = 64 * w + 32 * k + lane;
+                yV[o] = v[k] = vg::fe_fold(v0, v1, fb);
+                yAM[o] = m[k] = vg::fe_fold(m0, m1, fb);
+                yAV[o] = a[k] = vg::fe_fold(a0, a1, fb);
+            }
+            fe vo, vx, ao, ax, mo, mx;
+            pair_up(v[0], v[1], hi, 1, vo, vx);
+            pair_up(m[0], m[1], hi, 1, mo, mx);
+            pair_up(a[0], a[1], hi, 1, ao, ax);
+            pair_sums(vo, vx, ao, ax, mo, mx, hi, sb);
+        }
+        rg_sums_end(sa);
     }
-    round2_finish(sa, sb, sm, last, parts, counter, out_a, out_b, FOLD, ra, rb);
+    round2_finish(sa, sb, gacc, counter, out_a, out_b, FOLD, ra, rb);
 }
 
 // The phase's table build fused with its first two rounds (deferred mode,
-// paired rounds, tables above the group start).  A thread takes a quad of
-// consecutive keys, sums each key's edges as k_gather_keys does (a key with
-// more than LIGHT_MAX edges was summed beforehand by k_gather_long or
-// k_gather_heavy into tm / tv, read here), reads the quad's V entries and
-// runs k_round2's unfolded body on them: the addV and add_mult tables are
-// never written in full, and the pass after it starts from the folded
-// quarter.
+// paired rounds, tables above the group start).  A warp takes 128
+// consecutive keys, two pairs per lane, sums each key's edges as k_gather_keys
+// does (a key with more than LIGHT_MAX edges was summed beforehand by
+// k_gather_long or k_gather_heavy into tm / tv, read here), reads the V
+// entries (layer values, in F_p) and runs k_round2's unfolded body on them:
+// the addV and add_mult tables are never written in full, and the pass after
+// it starts from the folded half.
 struct GatherArgs {
     EdgeView e;
     BetaG bg;
@@ -1214,53 +1235,61 @@ struct GatherArgs {
 };
 
 template <int PH, int THREADS>
-__global__ void __launch_bounds__(THREADS) k_gather_round2(GatherArgs ga, const fe *__restrict__ xV, long nquads,
+__global__ void __launch_bounds__(THREADS, 512 / THREADS) k_gather_round2(GatherArgs ga, const fe *__restrict__ xV, long nquads,
                                                            const fe *__restrict__ rp, fe *__restrict__ yV,
                                                            fe *__restrict__ yAV, fe *__restrict__ yAM,
-                                                           fe *__restrict__ parts, unsigned *__restrict__ counter,
+                                                           unsigned long long *__restrict__ gacc, unsigned *__restrict__ counter,
                                                            fe *__restrict__ out_a, fe *__restrict__ out_b)
 {
-    __shared__ fe sm[6 * 32];
-    __shared__ bool last;
     const fe rb = rp[1];
     const fe vu = PH == 1 ? *ga.vu : vg::fe_zero();
+    const vg::fold_r fb = vg::fold_prep(rb);
+    const int lane = threadIdx.x & 31;
+    const bool hi = lane & 1;
+    const long nwarps = (long)gridDim.x * (THREADS / 32), w0 = (blockIdx.x * (long)THREADS + threadIdx.x) >> 5;
     fe sa[3] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero()}, sb[3] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nquads; i += (long)gridDim.x * blockDim.x) {
-        const long b = 4 * i;
-        fe v[4], a[4], m[4];
-        uint32_t off[5];
+    for (long w = w0; w < (nquads >> 5); w += nwarps) {
+        fe v[2], a[2], m[2];
 #pragma unroll
-        for (int k = 0; k < 5; ++k) off[k] = ga.e.off[b + k];
+        for (int h = 0; h < 2; ++h) {
+            const long k0 = 128 * w + 64 * h + 2 * lane;
+            fe av[2], am[2];
+            uint32_t s = ga.e.off[k0];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            v[k] = xV[b + k];
-            const uint32_t s = off[k], t = off[k + 1];
-            if (t - s > (uint32_t)LIGHT_MAX) {
-                m[k] = ga.tm[b + k];
-                a[k] = ga.tv[b + k];
-            } else if (PH == 0) {
-                fe am = vg::fe_zero(), av = vg::fe_zero();
-                for (uint32_t p = s; p < t; ++p) edge1(ga.e.tk[p], ga.e.g[p], ga.e.o[p], ga.bg, ga.prev, am, av);
-                m[k] = am;
-                a[k] = av;
-            } else {
-                fe q[4] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
-                unsigned used = 0;
-                for (uint32_t p = s; p < t; ++p) edge2(ga.e.tk[p], ga.e.g[p], ga.e.o[p], ga.bg, ga.bu, q, used);
-                phase2_out(q, used, vu, m[k], a[k]);
+            for (int k = 0; k < 2; ++k) {
+                const uint32_t t = ga.e.off[k0 + k + 1];
+                if (t - s > (uint32_t)LIGHT_MAX) {
+                    am[k] = ga.tm[k0 + k];
+                    av[k] = ga.tv[k0 + k];
+                } else if (PH == 0) {
+                    am[k] = av[k] = vg::fe_zero();
+                    for (uint32_t p = s; p < t; ++p) edge1(ga.e.tk[p], ga.e.g[p], ga.e.o[p], ga.bg, ga.prev, am[k], av[k]);
+                } else {
+                    fe q[4] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
+                    unsigned used = 0;
+                    for (uint32_t p = s; p < t; ++p) edge2(ga.e.tk[p], ga.e.g[p], ga.e.o[p], ga.bg, ga.bu, q, used);
+                    phase2_out(q, used, vu, am[k], av[k]);
+                }
+                s = t;
             }
+            fe v0, v1;
+            ld_pair(xV + k0, v0, v1);   // layer values: real parts
+            sa[0] = vg::fe_fma_real(sa[0], am[1] - am[0], v1.real + vg::P - v0.real);
+            sa[2] = vg::fe_fma_real(sa[2] + av[0], am[0], v0.real);
+            sa[1] = vg::fe_fma_real(sa[1] + av[1], am[1], v1.real);
+            const long o = 64 * w + 32 * h + lane;
+            yV[o] = v[h] = vg::fe_fold_real(v0.real, v1.real, fb);
+            yAM[o] = m[h] = vg::fe_fold(am[0], am[1], fb);
+            yAV[o] = a[h] = vg::fe_fold(av[0], av[1], fb);
         }
-        rg_sums(v[0], v[1], a[0], a[1], m[0], m[1], sa);
-        rg_sums(v[2], v[3], a[2], a[3], m[2], m[3], sa);
-        const fe v0 = fold<false>(v[0], v[1], rb), v1 = fold<false>(v[2], v[3], rb);
-        const fe a0 = fold<false>(a[0], a[1], rb), a1 = fold<false>(a[2], a[3], rb);
-        const fe m0 = fold<false>(m[0], m[1], rb), m1 = fold<false>(m[2], m[3], rb);
-        rg_sums<false>(v0, v1, a0, a1, m0, m1, sb);
-        yV[2 * i] = v0; yV[2 * i + 1] = v1;
-        yAV[2 * i] = a0; yAV[2 * i + 1] = a1;
-        yAM[2 * i] = m0; yAM[2 * i + 1] = m1;
+        fe vo, vx, ao, ax, mo, mx;
+        pair_up(v[0], v[1], hi, 1, vo, vx);
+        pair_up(m[0], m[1], hi, 1, mo, mx);
+        pair_up(a[0], a[1], hi, 1, ao, ax);
+        pair_sums(vo, vx, ao, ax, mo, mx, hi, sb);
     }
-    round2_finish(sa, sb, sm, last, parts, counter, out_a, out_b, false, vg::fe_zero(), rb);
+    rg_sums_end(sa);
+    round2_finish(sa, sb, gacc, counter, out_a, out_b, false, vg::fe_zero(), rb);
 }
 
 vg::fe tofe(vg_fe x) { return vg::fe_make(x.real, x.img); }
@@ -1355,7 +1384,6 @@ struct vg_circuit {
 struct RoundLaunch {
     int kind = 0;               // 0 k_round, 1 k_round2, 2 k_round_group, 3 k_gather_round2
     bool fold = false;
-    bool lazy = false;          // folds in the unreduced four-product form (VG_TUNE_LAZY_FOLD)
     int threads = 0;
     unsigned grid = 0;
     long count = 0;             // pairs (k_round), quads (k_round2), input entries (group)
@@ -1390,7 +1418,7 @@ struct vg_gkr {
     unsigned long long *acc = nullptr;   // 2 tables x 4 words x 2^max_bl
     fe *eq = nullptr;                    // half tables
     fe *rbuf = nullptr;                  // challenges (device copy)
-    fe *round_parts = nullptr;           // block partials of the round kernels (6 x 148 x 8 values)
+    unsigned long long *round_acc = nullptr;   // the round kernels' limb sums over the grid (grid_sum), zero between launches
     fe *round_out = nullptr;             // round sums (3) written by the last block
     unsigned *round_counter = nullptr;   // blocks finished, reset by the last one
     long eq_half = 0;
@@ -1894,7 +1922,8 @@ static int gkr_bind(vg_gkr *g, const vg_circuit *c)
         return vg_fail(VG_ERR_OOM, "vg_gkr: %s allocation failed", what);
     };
     long total = 0;
-    for (int i = 1; i < c->depth; ++i) total += c->L[i].n;
+    // each layer on a 256-byte boundary (the paired rounds load 32 bytes at a time)
+    for (int i = 1; i < c->depth; ++i) total += (c->L[i].n + 15) / 16 * 16;
     vg_ctx *x = g->ctx;
     if (total > g->vals_cap) {
         vg_release(x, g->vals_slab);
@@ -1908,7 +1937,7 @@ static int gkr_bind(vg_gkr *g, const vg_circuit *c)
     long off = 0;
     for (int i = 1; i < c->depth; ++i) {
         g->vals[i] = g->vals_slab + off;
-        off += c->L[i].n;
+        off += (c->L[i].n + 15) / 16 * 16;
     }
     const long N = 1L << c->max_bl;
     if (N > g->N_cap) {
@@ -1965,7 +1994,7 @@ extern "C" int vg_gkr_create(vg_ctx *ctx, const vg_circuit *c, vg_gkr **out)
         return vg_fail(VG_ERR_OOM, "vg_gkr_create: %s allocation failed", what);
     };
     if (cudaMalloc(&g->rbuf, 3 * 64 * sizeof(fe)) != cudaSuccess) return fail("challenges");
-    if (cudaMalloc(&g->round_parts, 6 * 148 * 8 * sizeof(fe)) != cudaSuccess) return fail("round partials");
+    if (cudaMalloc(&g->round_acc, LIMBS * 6 * 8) != cudaSuccess) return fail("round sums");
     if (cudaMalloc(&g->round_out, 16 * sizeof(fe)) != cudaSuccess) return fail("round sums");
     if (cudaMalloc(&g->round_counter, sizeof(unsigned)) != cudaSuccess) return fail("round counter");
     if (cudaMalloc(&g->vu, sizeof(fe)) != cudaSuccess) return fail("v_u");
@@ -1975,7 +2004,9 @@ extern "C" int vg_gkr_create(vg_ctx *ctx, const vg_circuit *c, vg_gkr **out)
         return fail("heavy partials");
     // on the context's stream: the streams are non-blocking, so a memset on
     // the legacy stream would not be ordered before the first round kernel
-    if (cudaMemsetAsync(g->round_counter, 0, sizeof(unsigned), ctx->stream) != cudaSuccess) return fail("round counter");
+    if (cudaMemsetAsync(g->round_counter, 0, sizeof(unsigned), ctx->stream) != cudaSuccess ||
+        cudaMemsetAsync(g->round_acc, 0, LIMBS * 6 * 8, ctx->stream) != cudaSuccess)
+        return fail("round counter");
     int rc = gkr_bind(g, c);
     if (rc != VG_OK) {
         vg_gkr_destroy(g);
@@ -2002,7 +2033,7 @@ extern "C" int vg_gkr_destroy(vg_gkr *g)
     cudaFree(g->acc);
     cudaFree(g->eq);
     cudaFree(g->rbuf);
-    cudaFree(g->round_parts);
+    cudaFree(g->round_acc);
     cudaFree(g->round_out);
     cudaFree(g->round_counter);
     cudaFree(g->vu);
@@ -2478,10 +2509,8 @@ static int rg_smem_attribute(int dev)
     if (dev >= (int)done.size()) done.resize(dev + 1, false);
     if (!done[dev]) {
         const int bytes = (int)(RG_SMEM_FE * sizeof(fe));
-        VG_CHECK_CUDA(cudaFuncSetAttribute(k_round_group<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        VG_CHECK_CUDA(cudaFuncSetAttribute(k_round_group<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        VG_CHECK_CUDA(cudaFuncSetAttribute(k_round_group<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        VG_CHECK_CUDA(cudaFuncSetAttribute(k_round_group<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        VG_CHECK_CUDA(cudaFuncSetAttribute(k_round_group<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        VG_CHECK_CUDA(cudaFuncSetAttribute(k_round_group<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
         done[dev] = true;
     }
     return VG_OK;
@@ -2494,39 +2523,31 @@ static int issue_launch(vg_gkr *g, const RoundLaunch &L, const fe *rp)
     vg_ctx *c = g->ctx;
     {
         ProfScope ps(c, L.kind == 3 ? KF_GATHER_ROUND : KF_ROUND, L.prof_bytes);
-        fe *pr = g->round_parts;
+        unsigned long long *pr = g->round_acc;
         unsigned *cnt = g->round_counter;
         if (L.kind == 0) {
-#define VG_ROUND_LAUNCH(TT, LZ)                                                                                      \
+#define VG_ROUND_LAUNCH(TT)                                                                                          \
     if (L.fold)                                                                                                       \
-        k_round<true, TT, LZ><<<L.grid, TT, 0, c->stream>>>(L.x[0], L.x[1], L.x[2], L.count, rp, L.y[0], L.y[1],     \
-                                                            L.y[2], pr, cnt, L.oa, L.ob, L.prev);                     \
+        k_round<true, TT><<<L.grid, TT, 0, c->stream>>>(L.x[0], L.x[1], L.x[2], L.count, rp, L.y[0], L.y[1], L.y[2], \
+                                                        pr, cnt, L.oa, L.ob, L.prev);                                 \
     else                                                                                                              \
-        k_round<false, TT, LZ><<<L.grid, TT, 0, c->stream>>>(L.x[0], L.x[1], L.x[2], L.count, rp, nullptr, nullptr,  \
-                                                             nullptr, pr, cnt, L.oa, L.ob, nullptr)
-#define VG_ROUND_LAUNCH_T(LZ)                     \
-    if (L.threads == 128) VG_ROUND_LAUNCH(128, LZ); \
-    else if (L.threads == 512) VG_ROUND_LAUNCH(512, LZ); \
-    else VG_ROUND_LAUNCH(256, LZ)
-            if (L.lazy) { VG_ROUND_LAUNCH_T(true); }
-            else { VG_ROUND_LAUNCH_T(false); }
-#undef VG_ROUND_LAUNCH_T
+        k_round<false, TT><<<L.grid, TT, 0, c->stream>>>(L.x[0], L.x[1], L.x[2], L.count, rp, nullptr, nullptr,      \
+                                                         nullptr, pr, cnt, L.oa, L.ob, nullptr)
+            if (L.threads == 128) VG_ROUND_LAUNCH(128);
+            else if (L.threads == 512) VG_ROUND_LAUNCH(512);
+            else VG_ROUND_LAUNCH(256);
 #undef VG_ROUND_LAUNCH
         } else if (L.kind == 1) {
-#define VG_ROUND2_LAUNCH(TT, LZ)                                                                                     \
+#define VG_ROUND2_LAUNCH(TT)                                                                                         \
     if (L.fold)                                                                                                       \
-        k_round2<true, TT, LZ><<<L.grid, TT, 0, c->stream>>>(L.x[0], L.x[1], L.x[2], L.count, rp, L.y[0], L.y[1],    \
-                                                             L.y[2], pr, cnt, L.oa, L.ob);                            \
+        k_round2<true, TT><<<L.grid, TT, 0, c->stream>>>(L.x[0], L.x[1], L.x[2], L.count, rp, L.y[0], L.y[1],        \
+                                                         L.y[2], pr, cnt, L.oa, L.ob);                                \
     else                                                                                                              \
-        k_round2<false, TT, LZ><<<L.grid, TT, 0, c->stream>>>(L.x[0], L.x[1], L.x[2], L.count, rp, L.y[0], L.y[1],   \
-                                                              L.y[2], pr, cnt, L.oa, L.ob)
-#define VG_ROUND2_LAUNCH_T(LZ)                     \
-    if (L.threads == 128) VG_ROUND2_LAUNCH(128, LZ); \
-    else if (L.threads == 512) VG_ROUND2_LAUNCH(512, LZ); \
-    else VG_ROUND2_LAUNCH(256, LZ)
-            if (L.lazy) { VG_ROUND2_LAUNCH_T(true); }
-            else { VG_ROUND2_LAUNCH_T(false); }
-#undef VG_ROUND2_LAUNCH_T
+        k_round2<false, TT><<<L.grid, TT, 0, c->stream>>>(L.x[0], L.x[1], L.x[2], L.count, rp, L.y[0], L.y[1],       \
+                                                          L.y[2], pr, cnt, L.oa, L.ob)
+            if (L.threads == 128) VG_ROUND2_LAUNCH(128);
+            else if (L.threads == 512) VG_ROUND2_LAUNCH(512);
+            else VG_ROUND2_LAUNCH(256);
 #undef VG_ROUND2_LAUNCH
         } else if (L.kind == 3) {
 #define VG_GR2_LAUNCH(TT, PH)                                                                                       \
@@ -2543,13 +2564,11 @@ static int issue_launch(vg_gkr *g, const RoundLaunch &L, const fe *rp)
         } else {
             RoundGroup G = L.G;
             G.r = rp;
-#define VG_GROUP_LAUNCH(LZ, SP)                                                                                      \
-    k_round_group<LZ, SP><<<L.grid, RG_THREADS, RG_SMEM_FE * sizeof(fe), c->stream>>>(                               \
+#define VG_GROUP_LAUNCH(SP)                                                                                          \
+    k_round_group<SP><<<L.grid, RG_THREADS, RG_SMEM_FE * sizeof(fe), c->stream>>>(                                   \
         L.x[0], L.x[1], L.x[2], L.count, G, L.y[0], L.y[1], L.y[2], g->rg_parts, g->round_counter, g->rec)
-            if (L.lazy && G.split3) VG_GROUP_LAUNCH(true, true);
-            else if (L.lazy) VG_GROUP_LAUNCH(true, false);
-            else if (G.split3) VG_GROUP_LAUNCH(false, true);
-            else VG_GROUP_LAUNCH(false, false);
+            if (G.split3) VG_GROUP_LAUNCH(true);
+            else VG_GROUP_LAUNCH(false);
 #undef VG_GROUP_LAUNCH
         }
     }
@@ -2630,7 +2649,7 @@ static int exec_pending(vg_gkr *g)
     key.push_back((uint64_t)lo);
     key.push_back((uint64_t)hi);
     for (const RoundLaunch &L : launches) {
-        key.push_back((uint64_t)L.kind | ((uint64_t)L.fold << 4) | ((uint64_t)L.lazy << 5) | ((uint64_t)L.threads << 16) |
+        key.push_back((uint64_t)L.kind | ((uint64_t)L.fold << 4) | ((uint64_t)L.threads << 16) |
                       ((uint64_t)L.grid << 32));
         key.push_back((uint64_t)L.count);
         for (int k = 0; k < 3; ++k) key.push_back((uint64_t)(uintptr_t)L.x[k]);
@@ -2653,7 +2672,7 @@ static int exec_pending(vg_gkr *g)
             key.push_back((uint64_t)a.bu.mask);
         }
     }
-    key.push_back((uint64_t)(uintptr_t)g->round_parts);
+    key.push_back((uint64_t)(uintptr_t)g->round_acc);
     key.push_back((uint64_t)(uintptr_t)g->round_counter);
     key.push_back((uint64_t)(uintptr_t)g->rg_parts);
     key.push_back((uint64_t)(uintptr_t)g->rec);
@@ -2712,14 +2731,13 @@ static int launch_round(vg_gkr *g, long n_in, bool fold, fe r, int slot, fe *o3,
     const long n_out = fold ? n_in / 2 : n_in;   // table length the sums are taken over
     const long npairs = n_out / 2;
     // threads per CTA from the device's tuning; the grid covers at most
-    // 148 x 2048 threads and at most 148 x 16 CTAs (the partials buffer holds
-    // 3 sums for each), looping beyond
+    // 148 x 2048 threads and at most 1024 CTAs (the limb sums' range), looping
+    // beyond
     RoundLaunch L;
     L.kind = 0;
     L.fold = fold;
-    L.lazy = vg_tune_value(c->device, VG_TUNE_LAZY_FOLD) != 0;
     L.threads = (int)vg_tune_value(c->device, VG_TUNE_ROUND_THREADS);
-    L.grid = std::min<unsigned>(grid_for(npairs, L.threads), std::min(148u * 16u, 148u * 2048u / (unsigned)L.threads));
+    L.grid = std::min<unsigned>(grid_for(npairs, L.threads), std::min(1024u, 148u * 2048u / (unsigned)L.threads));
     L.count = npairs;
     for (int k = 0; k < 3; ++k) {
         L.x[k] = g->cur[k];
@@ -2746,15 +2764,14 @@ static int launch_round2(vg_gkr *g, long n_in, bool fold, int slot)
 {
     vg_ctx *c = g->ctx;
     const long nquads = fold ? n_in / 8 : n_in / 4;
-    // at most 148 x 2048 threads and 148 x 8 CTAs (6 sums each in the partials buffer)
+    // a warp per 32 quads, at most the 512 threads per SM that are resident at once
     // the phase's pending table build runs inside its unfolded first pass
     const bool fused = g->gather_pending && !fold && n_in == g->gather_n;
     RoundLaunch L;
     L.kind = fused ? 3 : 1;
     L.fold = fold;
-    L.lazy = !fused && vg_tune_value(c->device, VG_TUNE_LAZY_FOLD) != 0;
     L.threads = (int)vg_tune_value(c->device, VG_TUNE_ROUND_THREADS);
-    L.grid = std::min<unsigned>(grid_for(nquads, L.threads), std::min(148u * 8u, 148u * 2048u / (unsigned)L.threads));
+    L.grid = std::min<unsigned>(grid_for(nquads, L.threads), 148u * 512u / (unsigned)L.threads);
     L.count = nquads;
     for (int k = 0; k < 3; ++k) {
         L.x[k] = g->cur[k];
@@ -2796,7 +2813,6 @@ static int group_rounds(vg_gkr *g)
     vg_ctx *c = g->ctx;
     RoundLaunch L;
     L.kind = 2;
-    L.lazy = vg_tune_value(c->device, VG_TUNE_LAZY_FOLD) != 0;
     RoundGroup &G = L.G;
     int cl = 0;
     while ((1L << cl) < g->pend_chunk) ++cl;
@@ -3014,7 +3030,9 @@ extern "C" int vg_gkr_round(vg_gkr *g, vg_fe previous_random, int current_bit, v
             g->round0_pending = false;
             return VG_OK;
         }
-        if (vg_tune_value(c->device, VG_TUNE_ROUND_FUSE) >= 2) {
+        // the paired pass loads entries two at a time: tables on 32-byte
+        // boundaries, as every table this library allocates is
+        if (vg_tune_value(c->device, VG_TUNE_ROUND_FUSE) >= 2 && ((uintptr_t)g->cur[0] & 31) == 0) {
             g->held = true;
             g->held_fold = fold;
             g->held_slot = g->rec_n;
@@ -3064,11 +3082,13 @@ int vg_gkr_tables_create(vg_ctx *ctx, long max_n, int max_records, vg_gkr **out)
         vg_gkr_destroy(g);
         return vg_fail(VG_ERR_OOM, "vg_gkr_tables_create: %s allocation failed", what);
     };
-    if (cudaMalloc(&g->round_parts, 6 * 148 * 8 * sizeof(fe)) != cudaSuccess) return fail("round partials");
+    if (cudaMalloc(&g->round_acc, LIMBS * 6 * 8) != cudaSuccess) return fail("round sums");
     if (cudaMalloc(&g->round_out, 16 * sizeof(fe)) != cudaSuccess) return fail("round sums");
     if (cudaMalloc(&g->round_counter, sizeof(unsigned)) != cudaSuccess) return fail("round counter");
     // ordered on the context's (non-blocking) stream before the first round
-    if (cudaMemsetAsync(g->round_counter, 0, sizeof(unsigned), ctx->stream) != cudaSuccess) return fail("round counter");
+    if (cudaMemsetAsync(g->round_counter, 0, sizeof(unsigned), ctx->stream) != cudaSuccess ||
+        cudaMemsetAsync(g->round_acc, 0, LIMBS * 6 * 8, ctx->stream) != cudaSuccess)
+        return fail("round counter");
     g->deferred = true;
     const int rc = vg_gkr_tables_reserve(g, max_n, max_records);
     if (rc != VG_OK) {
