@@ -48,6 +48,7 @@ struct vg_ctx {
     size_t scratch2_cap = 0;
     fe *partials = nullptr;  // block partial sums of reductions
     size_t partials_cap = 0;
+    unsigned long long *gsum = nullptr;   // grid_sum's limb sums and counter (vg_grid_scratch), zero between launches
     fe *pinned = nullptr;    // pinned host staging for small results
     size_t pinned_cap = 0;
     // pinned ring for uploads from pageable host memory (vg_h2d_staged)
@@ -133,6 +134,8 @@ int vg_scratch(vg_ctx *ctx, size_t bytes, void **p);
 int vg_scratch2(vg_ctx *ctx, size_t bytes, void **p);
 int vg_partials(vg_ctx *ctx, size_t n, fe **p);
 int vg_pinned(vg_ctx *ctx, size_t n, fe **p);
+// grid_sum's device words for the context's kernels (up to 14 values per sum)
+int vg_grid_scratch(vg_ctx *ctx, unsigned long long **gacc, unsigned **counter);
 int vg_twiddles(vg_ctx *ctx, fe root, int logn, const fe **lo, const fe **hi);
 bool vg_is_device_ptr(const void *p);
 

@@ -247,6 +247,7 @@ extern "C" int vg_ctx_destroy(vg_ctx *c)
     if (c->scratch) cudaFree(c->scratch);
     if (c->scratch2) cudaFree(c->scratch2);
     if (c->partials) cudaFree(c->partials);
+    if (c->gsum) cudaFree(c->gsum);
     if (c->pinned) cudaFreeHost(c->pinned);
     for (void *q : c->retired_pinned) cudaFreeHost(q);
     for (int k = 0; k < 2; ++k) {
@@ -407,6 +408,18 @@ int vg_pinned(vg_ctx *c, size_t n, fe **p)
     VG_TRY(vg_pinned_grow(c, &q, &c->pinned_cap, n * sizeof(fe)));
     c->pinned = (fe *)q;
     *p = c->pinned;
+    return VG_OK;
+}
+
+int vg_grid_scratch(vg_ctx *c, unsigned long long **gacc, unsigned **counter)
+{
+    constexpr size_t WORDS = LIMBS * 14;
+    if (!c->gsum) {
+        VG_TRY(vg_alloc(c, (void **)&c->gsum, (WORDS + 1) * 8));
+        VG_CHECK_CUDA(cudaMemsetAsync(c->gsum, 0, (WORDS + 1) * 8, c->stream));
+    }
+    *gacc = c->gsum;
+    *counter = (unsigned *)(c->gsum + WORDS);
     return VG_OK;
 }
 
