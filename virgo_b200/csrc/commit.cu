@@ -687,6 +687,7 @@ int vg_pc_prove_deferred(vg_pc *pc, const vg_fe *priv, int log_len, const vg_fe 
     for (int t = 0; t < nlevels; ++t) sets.push_back({pc->F(pc->levels[t].cw), pc->levels[t].n, pc->U(pc->levels[t].tree)});
     for (size_t b = 0; b < sets.size(); b += MAX_HASH_JOBS) {
         ChainJobs cj{};
+        cj.slices = 65;
         long total = 0;
         for (size_t k = b; k < sets.size() && k < b + MAX_HASH_JOBS; ++k) {
             const long nleaves = sets[k].n >> 1;

@@ -147,6 +147,10 @@ def main():
     # B[y, 2x + 3y] = A[x, y] puts A[(X + 3Y) % 5, X] at lane X + 5Y
     L.append("#define VG_KECCAK_RHO { " + ", ".join(str(rot[i % 5][i // 5]) for i in range(25)) + " }")
     L.append("#define VG_KECCAK_PI_SRC { " + ", ".join(str(((i % 5) + 3 * (i // 5)) % 5 + 5 * (i % 5)) for i in range(25)) + " }")
+    # the even and odd bits of the round constants (the two-lane formulation)
+    for name, odd in (("EVEN", 0), ("ODD", 1)):
+        half = [sum(((v >> (2 * j + odd)) & 1) << j for j in range(32)) for v in rc]
+        L.append("#define VG_KECCAK_RC_%s { " % name + ", ".join("0x%08xu" % v for v in half) + " }")
     L.append("")
     L.append("#define VG_KECCAK_ROUND32(RCL, RCH) { \\")
     L.extend(round32(rot, 0))

@@ -1,6 +1,7 @@
 // Hash kernels: batched 64-byte hashing, Merkle trees and the FRI leaf hash
 // chains.  All are integer-ALU bound (Keccak-f[1600]: 24 rounds of 64-bit
 // xor/and-not/rotate; SHA-256: 2 x 64 rounds of 32-bit ops).
+#include <algorithm>
 #include <mutex>
 #include "common.cuh"
 // 2^n, n < 32, for the multiply-pipe rotations (VG_MROT_*); filled per device
@@ -42,38 +43,6 @@ __global__ void k_hash64(const uint64_t *__restrict__ msgs, uint64_t *__restrict
 
 }  // namespace
 
-// ---- Merkle levels ----
-template <int KIND>
-__global__ void k_merkle_level(uint64_t *__restrict__ tree, long first, long count)
-{
-    // parents tree[first .. first+count) from children tree[2 first ..)
-    long j = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (j >= count) return;
-    long p = first + j;
-    uint64_t w[8], d[4];
-    load_digest2(tree + 8 * p, w);   // children 2p, 2p+1 are contiguous
-    vg::hash64<KIND>(w, d);
-    store_digest(tree + 4 * p, d);
-}
-
-// The top levels of a tree (at most 2 * MERKLE_TOP nodes below node 1) in one
-// CTA: each level waits for the one below with __syncthreads.
-template <int KIND>
-__global__ void k_merkle_top(uint64_t *__restrict__ tree, long width)
-{
-    for (long cnt = width; cnt >= 1; cnt >>= 1) {
-        for (long j = threadIdx.x; j < cnt; j += blockDim.x) {
-            long p = cnt + j;
-            uint64_t w[8], d[4];
-            load_digest2(tree + 8 * p, w);
-            vg::hash64<KIND>(w, d);
-            store_digest(tree + 4 * p, d);
-        }
-        __threadfence_block();
-        __syncthreads();
-    }
-}
-
 template <int KIND>
 __global__ void k_fill_pad(uint64_t *__restrict__ tree, long from, long to)
 {
@@ -86,42 +55,29 @@ __global__ void k_fill_pad(uint64_t *__restrict__ tree, long from, long to)
 
 // ---- leaf hash chains ----
 // Leaf k of a codeword set with per-slice length n: h = 0; for s:
-// h = H(c[s][k] || c[s][k + n/2] || h).  One thread per leaf; a warp reads
-// 32 consecutive k of one slice, i.e. 512 contiguous bytes per load.
-template <int KIND, int T>
-__global__ void __launch_bounds__(T) k_leaf_chain(const fe *__restrict__ c, int n_slices, long n,
-                                                 uint64_t *__restrict__ leaves)
+// h = H(c[s][k] || c[s][k + n/2] || h).  Several sets in one launch: chain t is
+// leaf t - begin of the job whose range holds t.  One thread per chain (a
+// warp reads 32 consecutive k of one slice, 512 contiguous bytes per load; the
+// next slice's pair is loaded before the current hash), except the chains from
+// thread_chains on, which take a pair of lanes each (vg_leaf_chains chooses).
+__device__ __forceinline__ int chain_job(const ChainJobs &jobs, long t)
 {
-    const long half = n >> 1;
-    long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (k >= half) return;
-    uint64_t h[4] = {0, 0, 0, 0};
-    for (int s = 0; s < n_slices; ++s) {
-        fe a = c[(long)s * n + k], b = c[(long)s * n + k + half];
-        uint64_t w[8] = {a.img, a.real, b.img, b.real, h[0], h[1], h[2], h[3]};
-        vg::hash64<KIND>(w, h);
-    }
-    store_digest(leaves + 4 * k, h);
-}
-
-// ---- batched forms: every leaf chain and every Merkle tree of a proof ----
-// Leaf chains of several codeword sets in one launch: thread t serves leaf
-// t - begin of the job whose range holds t.  The next slice's pair is loaded
-// before the current hash so the loads overlap the permutation.
-template <int KIND, int T, int ROT>
-__global__ void __launch_bounds__(T) k_leaf_chains(ChainJobs jobs)
-{
-    const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (t >= jobs.total) return;
     int q = 0;
     while (q + 1 < jobs.count && t >= jobs.j[q + 1].begin) ++q;
+    return q;
+}
+
+template <int KIND, int ROT>
+__device__ __forceinline__ void thread_chain(const ChainJobs &jobs, long t)
+{
+    const int q = chain_job(jobs, t);
     const fe *__restrict__ c = jobs.j[q].cw;
     const long n = jobs.j[q].n, half = n >> 1, k = t - jobs.j[q].begin;
     uint64_t h[4] = {0, 0, 0, 0};
     fe a = c[k], b = c[k + half];
-    for (int s = 0; s < 65; ++s) {
+    for (int s = 0; s < jobs.slices; ++s) {
         fe na = a, nb = b;
-        if (s + 1 < 65) {
+        if (s + 1 < jobs.slices) {
             na = c[(long)(s + 1) * n + k];
             nb = c[(long)(s + 1) * n + k + half];
         }
@@ -131,6 +87,52 @@ __global__ void __launch_bounds__(T) k_leaf_chains(ChainJobs jobs)
         b = nb;
     }
     store_digest(jobs.j[q].leaves + 4 * k, h);
+}
+
+// a chain on lanes 2j and 2j + 1; t at most total - 1 (every lane takes part
+// in the shuffles), stored when `active`
+__device__ __forceinline__ void pair_chain(const ChainJobs &jobs, long t, bool active)
+{
+    const bool odd = threadIdx.x & 1;
+    const int q = chain_job(jobs, t);
+    const fe *__restrict__ c = jobs.j[q].cw;
+    const long n = jobs.j[q].n, half = n >> 1, k = t - jobs.j[q].begin;
+    uint32_t s25[25];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s25[i] = 0;
+    fe a = c[k], b = c[k + half];
+    for (int s = 0; s < jobs.slices; ++s) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s25[4 + i] = s25[i];
+        s25[0] = vg::pair_half(a.img, odd);
+        s25[1] = vg::pair_half(a.real, odd);
+        s25[2] = vg::pair_half(b.img, odd);
+        s25[3] = vg::pair_half(b.real, odd);
+        if (s + 1 < jobs.slices) {
+            a = c[(long)(s + 1) * n + k];
+            b = c[(long)(s + 1) * n + k + half];
+        }
+        vg::sha3_256_64_pair(s25, odd);
+    }
+    uint32_t *out = reinterpret_cast<uint32_t *>(jobs.j[q].leaves + 4 * k) + (odd ? 1 : 0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t w = vg::pair_word(s25[i], odd);
+        if (active) out[2 * i] = w;
+    }
+}
+
+template <int KIND, int T, int ROT>
+__global__ void __launch_bounds__(T, 768 / T) k_leaf_chains(const __grid_constant__ ChainJobs jobs)
+{
+    const long nt = (jobs.thread_chains + T - 1) / T;   // CTAs of one thread per chain
+    if (blockIdx.x < nt) {
+        const long t = blockIdx.x * (long)T + threadIdx.x;
+        if (t < jobs.thread_chains) thread_chain<KIND, ROT>(jobs, t);
+    } else if (KIND == VG_HASH_SHA3_256 && ROT == 3) {
+        const long t = jobs.thread_chains + (blockIdx.x - nt) * (T / 2) + (threadIdx.x >> 1);
+        pair_chain(jobs, min(t, jobs.total - 1), t < jobs.total);
+    }
 }
 
 // ---- leaf chains, one warp per chain (SHA3-256 only) ----
@@ -173,22 +175,13 @@ __device__ __forceinline__ void warp_chain(const fe *__restrict__ c, int n_slice
 
 constexpr int WARP_CHAIN_THREADS = 128;
 
-__global__ void __launch_bounds__(WARP_CHAIN_THREADS) k_leaf_chains_warp(ChainJobs jobs)
+__global__ void __launch_bounds__(WARP_CHAIN_THREADS) k_leaf_chains_warp(const __grid_constant__ ChainJobs jobs)
 {
     const long w = ((long)blockIdx.x * WARP_CHAIN_THREADS + threadIdx.x) >> 5;
     if (w >= jobs.total) return;   // whole warps
-    int q = 0;
-    while (q + 1 < jobs.count && w >= jobs.j[q + 1].begin) ++q;
+    const int q = chain_job(jobs, w);
     const long k = w - jobs.j[q].begin;
-    warp_chain(jobs.j[q].cw, 65, jobs.j[q].n, k, jobs.j[q].leaves + 4 * k);
-}
-
-__global__ void __launch_bounds__(WARP_CHAIN_THREADS) k_leaf_chain_warp(const fe *__restrict__ c, int n_slices, long n,
-                                                                       uint64_t *__restrict__ leaves)
-{
-    const long k = ((long)blockIdx.x * WARP_CHAIN_THREADS + threadIdx.x) >> 5;
-    if (k >= (n >> 1)) return;   // whole warps
-    warp_chain(c, n_slices, n, k, leaves + 4 * k);
+    warp_chain(jobs.j[q].cw, jobs.slices, jobs.j[q].n, k, jobs.j[q].leaves + 4 * k);
 }
 
 static unsigned warp_chain_grid(long chains)
@@ -204,16 +197,16 @@ static bool use_warp_chains(vg_ctx *c, long chains)
 }
 
 // One Merkle level (parents of height `height`) of every tree that still has
-// more than MERKLE_TOP parents there.
+// more than MERKLE_SUB_MAX parents there, one thread per parent.
 template <int KIND>
-__global__ void __launch_bounds__(HASH_THREADS) k_merkle_levels(TreeJobs jobs, int height, long total)
+__global__ void __launch_bounds__(HASH_THREADS) k_merkle_levels(const __grid_constant__ TreeJobs jobs, int height, long total)
 {
     long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (t >= total) return;
     int q = 0;
     for (; q < jobs.count; ++q) {
         const long cnt = jobs.t[q].nleaves >> height;
-        if (cnt <= MERKLE_TOP) continue;
+        if (cnt <= MERKLE_SUB_MAX) continue;
         if (t < cnt) break;
         t -= cnt;
     }
@@ -225,25 +218,87 @@ __global__ void __launch_bounds__(HASH_THREADS) k_merkle_levels(TreeJobs jobs, i
     store_digest(jobs.t[q].tree + 4 * p, d);
 }
 
-// The top MERKLE_TOP parents and above of every tree, one CTA per tree; the
-// root is also copied to roots[tree].
+// Subtrees: a CTA hashes 64 neighbouring parents of a tree's next level, then
+// their 32 parents, up to seven levels, the digests of a level staying in
+// shared memory for the next.  The levels are a chain of dependent hashes, so
+// what counts is one hash's latency: SHA3 runs on pairs of lanes.  Trees of up
+// to 2^14 leaves take two launches of 14 such levels where one CTA took 4.6 us
+// and more for each of the top nine and a launch went to each level below.
+struct SubJobs {
+    struct {
+        uint64_t *tree;
+        long cnt;       // parents of the first level
+        int begin;      // first CTA
+    } t[MAX_HASH_JOBS];
+    int count;
+    uint64_t *roots;    // 4 words per tree, or null
+    int root_at[MAX_HASH_JOBS];
+};
 template <int KIND>
-__global__ void __launch_bounds__(MERKLE_TOP) k_merkle_tops(TreeJobs jobs, uint64_t *__restrict__ roots)
+__global__ void __launch_bounds__(2 * SUB_WIDTH) k_merkle_sub(const __grid_constant__ SubJobs J)
 {
-    const TreeJob J = jobs.t[blockIdx.x];
-    uint64_t *tree = J.tree;
-    for (long cnt = J.nleaves >> 1 < MERKLE_TOP ? J.nleaves >> 1 : MERKLE_TOP; cnt >= 1; cnt >>= 1) {
-        for (long j = threadIdx.x; j < cnt; j += blockDim.x) {
-            const long p = cnt + j;
+    // two levels' digests in turn: SHA3 as (even, odd) halves of 4 words
+    __shared__ __align__(16) uint32_t sd[2][SUB_WIDTH][8];
+    const int t = threadIdx.x;
+    int q = 0;
+    while (q + 1 < J.count && (int)blockIdx.x >= J.t[q + 1].begin) ++q;
+    uint64_t *tree = J.t[q].tree;
+    const long first = ((long)blockIdx.x - J.t[q].begin) * SUB_WIDTH;   // of this CTA among the level's parents
+    long cnt = J.t[q].cnt;                                              // the level's parents
+    int own = (int)min((long)SUB_WIDTH, cnt);                           // of them this CTA's
+    for (int lvl = 0; own >= 1; ++lvl, own >>= 1, cnt >>= 1) {
+        const long p0 = cnt + (first >> lvl);   // first parent's node
+        if (KIND == VG_HASH_SHA3_256) {
+            const bool odd = t & 1;
+            const int j = t >> 1;
+            if ((t & ~31) < 2 * own) {   // whole warps
+                const int jj = min(j, own - 1);
+                uint32_t a[25];
+                if (lvl == 0) {
+                    uint64_t w[8];
+                    load_digest2(tree + 8 * (p0 + jj), w);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) a[i] = vg::pair_half(w[i], odd);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) a[i] = sd[lvl & 1][2 * jj + (i >> 2)][2 * (i & 3) + odd];
+                }
+                vg::sha3_256_64_pair(a, odd);
+                uint32_t *out = reinterpret_cast<uint32_t *>(tree + 4 * (p0 + jj)) + (odd ? 1 : 0);
+                uint32_t w32[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w32[i] = vg::pair_word(a[i], odd);
+                if (j < own) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) out[2 * i] = w32[i];
+                    if (cnt == 1 && J.roots) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            reinterpret_cast<uint32_t *>(J.roots + 4 * J.root_at[q])[2 * i + odd] = w32[i];
+                    }
+                }
+                if (j < own) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) sd[~lvl & 1][j][2 * i + odd] = a[i];
+                }
+            }
+        } else if (t < own) {
             uint64_t w[8], d[4];
-            load_digest2(tree + 8 * p, w);
+            if (lvl == 0) {
+                load_digest2(tree + 8 * (p0 + t), w);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) w[i] = reinterpret_cast<const uint64_t *>(sd[lvl & 1][2 * t + (i >> 2)])[i & 3];
+            }
             vg::hash64<KIND>(w, d);
-            store_digest(tree + 4 * p, d);
+            store_digest(tree + 4 * (p0 + t), d);
+            if (cnt == 1 && J.roots)
+                for (int i = 0; i < 4; ++i) J.roots[4 * J.root_at[q] + i] = d[i];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) reinterpret_cast<uint64_t *>(sd[~lvl & 1][t])[i] = d[i];
         }
-        __threadfence_block();
         __syncthreads();
     }
-    if (threadIdx.x < 4) roots[4 * blockIdx.x + threadIdx.x] = tree[4 + threadIdx.x];
 }
 
 // fills vg_pow2c on the current device, once per device
@@ -262,29 +317,53 @@ static int pow2_table(int dev)
     return VG_OK;
 }
 
-int vg_leaf_chains(vg_ctx *c, const ChainJobs &jobs)
+// How many of `chains` SHA3 chains get a thread each.  Every scheduler of the
+// chip (4 per SM) runs whole warps, and one warp of 32 chains keeps it busy for
+// a full chain's time, so a last round of warps on some of them costs as much
+// as one on all.  Up to half a warp per scheduler is left over as pairs of
+// lanes instead, whose warps take about half as long: 98304 chains (5.2 warps
+// per scheduler) 1.69 -> 1.57 ms, 24576 (1.3) 571 -> 436 us, 2048 569 -> 169
+// us.  From six warps on the rounds average out.
+constexpr long SCHEDULERS = 148 * 4;
+static long thread_chains(long chains)
 {
-    if (jobs.total < 1) return VG_OK;
+    const long warps = (chains + 31) / 32, full = warps / SCHEDULERS, rest = warps % SCHEDULERS;
+    return full >= 6 || 2 * rest > SCHEDULERS ? chains : full * SCHEDULERS * 32;
+}
+
+int vg_leaf_chains(vg_ctx *c, const ChainJobs &jobs_in)
+{
+    if (jobs_in.total < 1) return VG_OK;
+    ChainJobs jobs = jobs_in;
     double bytes = 0;
-    for (int q = 0; q < jobs.count; ++q) bytes += 16.0 * 65.0 * (double)jobs.j[q].n + 32.0 * (double)(jobs.j[q].n >> 1);
+    for (int q = 0; q < jobs.count; ++q)
+        bytes += 16.0 * jobs.slices * (double)jobs.j[q].n + 32.0 * (double)(jobs.j[q].n >> 1);
     ProfScope ps(c, KF_LEAF_CHAIN, bytes);
     if (use_warp_chains(c, jobs.total)) {
         k_leaf_chains_warp<<<warp_chain_grid(jobs.total), WARP_CHAIN_THREADS, 0, c->stream>>>(jobs);
     } else {
-        const int T = (int)vg_tune_value(c->device, VG_TUNE_LEAF_THREADS);
+        int T = (int)vg_tune_value(c->device, VG_TUNE_LEAF_THREADS);
         const int rot = c->hash_kind == VG_HASH_SHA3_256 ? (int)vg_tune_value(c->device, VG_TUNE_LEAF_ROT) : 0;
         if (rot == 1 || rot == 2) VG_TRY(pow2_table(c->device));
+        jobs.thread_chains = rot == 3 ? thread_chains(jobs.total) : jobs.total;
+        // one warp more or less per scheduler matters while there are few: small
+        // CTAs spread them (131072 chains 2.26 ms in CTAs of 256, 1.99 of 64);
+        // CTAs of 128 put one warp of threads on every scheduler of an SM
+        if (jobs.thread_chains < jobs.total) T = 128;
+        else if (jobs.total < 24 * SCHEDULERS * 32) T = 64;
+        const long rest = jobs.total - jobs.thread_chains;
+        const unsigned grid = (unsigned)((jobs.thread_chains + T - 1) / T + (rest + T / 2 - 1) / (T / 2));
 #define VG_CHAINS_LAUNCH(TT)                                                                                    \
     if (c->hash_kind == VG_HASH_SHA256)                                                                          \
-        k_leaf_chains<VG_HASH_SHA256, TT, 0><<<grid_for(jobs.total, TT), TT, 0, c->stream>>>(jobs);             \
+        k_leaf_chains<VG_HASH_SHA256, TT, 0><<<grid, TT, 0, c->stream>>>(jobs);                                 \
     else if (rot == 1)                                                                                           \
-        k_leaf_chains<VG_HASH_SHA3_256, TT, 1><<<grid_for(jobs.total, TT), TT, 0, c->stream>>>(jobs);          \
+        k_leaf_chains<VG_HASH_SHA3_256, TT, 1><<<grid, TT, 0, c->stream>>>(jobs);                              \
     else if (rot == 2)                                                                                           \
-        k_leaf_chains<VG_HASH_SHA3_256, TT, 2><<<grid_for(jobs.total, TT), TT, 0, c->stream>>>(jobs);          \
+        k_leaf_chains<VG_HASH_SHA3_256, TT, 2><<<grid, TT, 0, c->stream>>>(jobs);                              \
     else if (rot == 3)                                                                                           \
-        k_leaf_chains<VG_HASH_SHA3_256, TT, 3><<<grid_for(jobs.total, TT), TT, 0, c->stream>>>(jobs);          \
+        k_leaf_chains<VG_HASH_SHA3_256, TT, 3><<<grid, TT, 0, c->stream>>>(jobs);                              \
     else                                                                                                         \
-        k_leaf_chains<VG_HASH_SHA3_256, TT, 0><<<grid_for(jobs.total, TT), TT, 0, c->stream>>>(jobs)
+        k_leaf_chains<VG_HASH_SHA3_256, TT, 0><<<grid, TT, 0, c->stream>>>(jobs)
         if (T == 64) VG_CHAINS_LAUNCH(64);
         else if (T == 256) VG_CHAINS_LAUNCH(256);
         else VG_CHAINS_LAUNCH(128);
@@ -301,7 +380,7 @@ int vg_merkle_trees(vg_ctx *c, const TreeJobs &jobs, uint64_t *roots_dev)
         long total = 0;
         for (int q = 0; q < jobs.count; ++q) {
             const long cnt = jobs.t[q].nleaves >> height;
-            if (cnt > MERKLE_TOP) total += cnt;
+            if (cnt > MERKLE_SUB_MAX) total += cnt;
         }
         if (total == 0) break;
         ProfScope ps(c, KF_MERKLE, 96.0 * (double)total);
@@ -311,12 +390,30 @@ int vg_merkle_trees(vg_ctx *c, const TreeJobs &jobs, uint64_t *roots_dev)
             k_merkle_levels<VG_HASH_SHA3_256><<<grid_for(total, HASH_THREADS), HASH_THREADS, 0, c->stream>>>(jobs, height, total);
         VG_LAUNCHED(c);
     }
-    ProfScope ps(c, KF_MERKLE, 96.0 * 2.0 * MERKLE_TOP * jobs.count);
-    if (c->hash_kind == VG_HASH_SHA256)
-        k_merkle_tops<VG_HASH_SHA256><<<jobs.count, MERKLE_TOP, 0, c->stream>>>(jobs, roots_dev);
-    else
-        k_merkle_tops<VG_HASH_SHA3_256><<<jobs.count, MERKLE_TOP, 0, c->stream>>>(jobs, roots_dev);
-    VG_LAUNCHED(c);
+    // the levels below, seven at a time
+    long cnt[MAX_HASH_JOBS];
+    for (int q = 0; q < jobs.count; ++q) cnt[q] = std::min(jobs.t[q].nleaves >> 1, MERKLE_SUB_MAX);
+    for (;;) {
+        SubJobs J{};
+        J.roots = roots_dev;
+        int ctas = 0;
+        double parents = 0;
+        for (int q = 0; q < jobs.count; ++q) {
+            if (cnt[q] < 1) continue;
+            J.t[J.count] = {jobs.t[q].tree, cnt[q], ctas};
+            J.root_at[J.count++] = q;
+            ctas += (int)((cnt[q] + SUB_WIDTH - 1) / SUB_WIDTH);
+            parents += 2.0 * (double)cnt[q];
+            cnt[q] >>= SUB_LEVELS;
+        }
+        if (!ctas) break;
+        ProfScope ps(c, KF_MERKLE, 96.0 * parents);
+        if (c->hash_kind == VG_HASH_SHA256)
+            k_merkle_sub<VG_HASH_SHA256><<<ctas, 2 * SUB_WIDTH, 0, c->stream>>>(J);
+        else
+            k_merkle_sub<VG_HASH_SHA3_256><<<ctas, 2 * SUB_WIDTH, 0, c->stream>>>(J);
+        VG_LAUNCHED(c);
+    }
     return VG_OK;
 }
 
@@ -324,49 +421,20 @@ int vg_merkle_trees(vg_ctx *c, const TreeJobs &jobs, uint64_t *roots_dev)
 int vg_merkle_build(vg_ctx *c, uint64_t *tree, long n_leaves_padded)
 {
     // leaves already in tree[sz .. 2 sz); builds nodes 1 .. sz-1
-    const long TOP = 1024;
-    long cnt = n_leaves_padded >> 1;
-    while (cnt > TOP) {
-        ProfScope ps(c, KF_MERKLE, 96.0 * (double)cnt);
-        if (c->hash_kind == VG_HASH_SHA256)
-            k_merkle_level<VG_HASH_SHA256><<<grid_for(cnt, HASH_THREADS), HASH_THREADS, 0, c->stream>>>(tree, cnt, cnt);
-        else
-            k_merkle_level<VG_HASH_SHA3_256><<<grid_for(cnt, HASH_THREADS), HASH_THREADS, 0, c->stream>>>(tree, cnt, cnt);
-        VG_LAUNCHED(c);
-        cnt >>= 1;
-    }
-    if (cnt >= 1) {
-        ProfScope ps(c, KF_MERKLE, 96.0 * (double)(2 * cnt));
-        if (c->hash_kind == VG_HASH_SHA256)
-            k_merkle_top<VG_HASH_SHA256><<<1, 512, 0, c->stream>>>(tree, cnt);
-        else
-            k_merkle_top<VG_HASH_SHA3_256><<<1, 512, 0, c->stream>>>(tree, cnt);
-        VG_LAUNCHED(c);
-    }
-    return VG_OK;
+    TreeJobs j{};
+    j.t[0] = {tree, n_leaves_padded};
+    j.count = 1;
+    return vg_merkle_trees(c, j, nullptr);
 }
 
 int vg_leaf_chain_dev(vg_ctx *c, const fe *cw, int n_slices, long n, uint64_t *leaves)
 {
-    long half = n >> 1;
-    if (half < 1) return VG_OK;
-    ProfScope ps(c, KF_LEAF_CHAIN, 16.0 * (double)n_slices * (double)n + 32.0 * (double)half);
-    if (use_warp_chains(c, half)) {
-        k_leaf_chain_warp<<<warp_chain_grid(half), WARP_CHAIN_THREADS, 0, c->stream>>>(cw, n_slices, n, leaves);
-    } else {
-        const int T = (int)vg_tune_value(c->device, VG_TUNE_LEAF_THREADS);
-#define VG_CHAIN_LAUNCH(TT)                                                                                           \
-    if (c->hash_kind == VG_HASH_SHA256)                                                                                \
-        k_leaf_chain<VG_HASH_SHA256, TT><<<grid_for(half, TT), TT, 0, c->stream>>>(cw, n_slices, n, leaves);          \
-    else                                                                                                               \
-        k_leaf_chain<VG_HASH_SHA3_256, TT><<<grid_for(half, TT), TT, 0, c->stream>>>(cw, n_slices, n, leaves)
-        if (T == 64) VG_CHAIN_LAUNCH(64);
-        else if (T == 256) VG_CHAIN_LAUNCH(256);
-        else VG_CHAIN_LAUNCH(128);
-#undef VG_CHAIN_LAUNCH
-    }
-    VG_LAUNCHED(c);
-    return VG_OK;
+    ChainJobs j{};
+    j.j[0] = {cw, n, leaves, 0};
+    j.count = 1;
+    j.total = n >> 1;
+    j.slices = n_slices;
+    return vg_leaf_chains(c, j);
 }
 
 extern "C" int vg_hash64(vg_ctx *c, const void *msgs, void *digests, long n)

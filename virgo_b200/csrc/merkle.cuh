@@ -8,19 +8,23 @@ int vg_merkle_build(vg_ctx *c, uint64_t *tree, long n_leaves_padded);
 // Leaf hash chains of a slice-major codeword set (see vg_leaf_chain).
 int vg_leaf_chain_dev(vg_ctx *c, const fe *cw, int n_slices, long n, uint64_t *leaves);
 
-// Batched leaf chains (65 slices each) and Merkle trees of one proof.
+// Batched leaf chains and Merkle trees of one proof.
 constexpr int MAX_HASH_JOBS = 16;
-constexpr int MERKLE_TOP = 256;   // parents per tree left to the one-CTA top pass
+// A tree's levels with at most this many parents are built by CTAs that own a
+// subtree of SUB_WIDTH parents and its levels above (vg_merkle_trees)
+constexpr long MERKLE_SUB_MAX = 8192;
+constexpr int SUB_WIDTH = 64, SUB_LEVELS = 7;
 struct ChainJob {
-    const fe *cw;       // slice-major codeword set, 65 slices of n
+    const fe *cw;       // slice-major codeword set, slices of n
     long n;
     uint64_t *leaves;   // n / 2 digests
     long begin;         // first thread of this job
 };
 struct ChainJobs {
     ChainJob j[MAX_HASH_JOBS];
-    int count;
-    long total;   // threads = sum of n / 2
+    int count, slices;
+    long total;   // chains = sum of n / 2
+    long thread_chains;   // of those, the first ones hashed by one thread each; the others by two lanes each
 };
 struct TreeJob {
     uint64_t *tree;   // heap-ordered, leaves at [nleaves, 2 nleaves)
@@ -31,5 +35,5 @@ struct TreeJobs {
     int count;
 };
 int vg_leaf_chains(vg_ctx *c, const ChainJobs &jobs);
-// Builds every tree; roots_dev receives 4 words per tree, in job order.
+// Builds every tree; roots_dev (or null) receives 4 words per tree of at least two leaves, in job order.
 int vg_merkle_trees(vg_ctx *c, const TreeJobs &jobs, uint64_t *roots_dev);
