@@ -699,7 +699,7 @@ int vg_pc_prove_deferred(vg_pc *pc, const vg_fe *priv, int log_len, const vg_fe 
     }
     for (size_t b = 0; b < sets.size(); b += MAX_HASH_JOBS) {
         TreeJobs tj{};
-        for (size_t k = b; k < sets.size() && k < b + MAX_HASH_JOBS; ++k) tj.t[tj.count++] = {sets[k].tree, sets[k].n >> 1};
+        for (size_t k = b; k < sets.size() && k < b + MAX_HASH_JOBS; ++k) tj.t[tj.count++] = {sets[k].tree, sets[k].n >> 1, sets[k].n >> 1};
         VG_TRY(vg_merkle_trees(c, tj, pc->U(pc->roots) + 4 * b));
     }
 

@@ -2,6 +2,7 @@
 // chains.  All are integer-ALU bound (Keccak-f[1600]: 24 rounds of 64-bit
 // xor/and-not/rotate; SHA-256: 2 x 64 rounds of 32-bit ops).
 #include <algorithm>
+#include <cstring>
 #include <mutex>
 #include "common.cuh"
 // 2^n, n < 32, for the multiply-pipe rotations (VG_MROT_*); filled per device
@@ -10,6 +11,8 @@
 static __constant__ uint32_t vg_pow2c[32];
 #include "hash.cuh"
 #include "merkle.cuh"
+
+void virgo_hash64_kind(int kind, const void *src, void *dst);   // host/src/hash_host.cpp
 
 namespace {
 
@@ -43,14 +46,40 @@ __global__ void k_hash64(const uint64_t *__restrict__ msgs, uint64_t *__restrict
 
 }  // namespace
 
-template <int KIND>
-__global__ void k_fill_pad(uint64_t *__restrict__ tree, long from, long to)
+// ---- Merkle trees ----
+// Padding leaves are all H(0^64), so a subtree of 2^h of them has one digest
+// per height; a ragged tree's levels write it where such nodes are instead of
+// hashing (70001 leaves: 70 thousand hashes, not 192 thousand).  The digests
+// are constants of the hash, formed on the host.
+static void pad_digests(int kind, uint64_t *pad)
 {
-    long i = from + blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (i >= to) return;
-    uint64_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0}, d[4];
-    vg::hash64<KIND>(w, d);
-    store_digest(tree + 4 * i, d);
+    uint64_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int h = 0; h < PAD_HEIGHTS; ++h) {
+        virgo_hash64_kind(kind, w, pad + 4 * h);
+        for (int i = 0; i < 8; ++i) w[i] = pad[4 * h + (i & 3)];
+    }
+}
+static const uint64_t *pad_table(int kind)
+{
+    struct Table {
+        uint64_t d[2][4 * PAD_HEIGHTS];
+        Table()
+        {
+            pad_digests(0, d[0]);
+            pad_digests(1, d[1]);
+        }
+    };
+    static const Table t;
+    return t.d[kind == VG_HASH_SHA256 ? 1 : 0];
+}
+
+// tree[0] cleared, the leaves and the padding after them: 16 bytes per thread
+__global__ void k_tree_leaves(const ulonglong2 *leaves, long n, long size, ulonglong2 p0, ulonglong2 p1, ulonglong2 *tree)
+{
+    const long stride = (long)gridDim.x * blockDim.x;
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < 2 * size; i += stride)
+        tree[2 * size + i] = i < 2 * n ? leaves[i] : (i & 1 ? p1 : p0);
+    if (blockIdx.x == 0 && threadIdx.x < 2) tree[threadIdx.x] = make_ulonglong2(0, 0);
 }
 
 // ---- leaf hash chains ----
@@ -213,8 +242,13 @@ __global__ void __launch_bounds__(HASH_THREADS) k_merkle_levels(const __grid_con
     if (q >= jobs.count) return;
     const long p = (jobs.t[q].nleaves >> height) + t;
     uint64_t w[8], d[4];
-    load_digest2(jobs.t[q].tree + 8 * p, w);
-    vg::hash64<KIND>(w, d);
+    if (jobs.padded && (t << height) >= jobs.t[q].nreal) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[i] = jobs.pad[4 * height + i];
+    } else {
+        load_digest2(jobs.t[q].tree + 8 * p, w);
+        vg::hash64<KIND>(w, d);
+    }
     store_digest(jobs.t[q].tree + 4 * p, d);
 }
 
@@ -422,7 +456,7 @@ int vg_merkle_build(vg_ctx *c, uint64_t *tree, long n_leaves_padded)
 {
     // leaves already in tree[sz .. 2 sz); builds nodes 1 .. sz-1
     TreeJobs j{};
-    j.t[0] = {tree, n_leaves_padded};
+    j.t[0] = {tree, n_leaves_padded, n_leaves_padded};
     j.count = 1;
     return vg_merkle_trees(c, j, nullptr);
 }
@@ -454,16 +488,21 @@ extern "C" int vg_merkle_tree(vg_ctx *c, const vg_digest *leaves, long n, vg_dig
     if (!c || !leaves || !tree || n < 1) return vg_fail(VG_ERR_ARG, "vg_merkle_tree: bad argument");
     long sz = 1;
     while (sz < n) sz <<= 1;
-    VG_CHECK_CUDA(cudaMemsetAsync(tree, 0, 2 * sz * sizeof(vg_digest), c->stream));
-    VG_CHECK_CUDA(cudaMemcpyAsync(tree + sz, leaves, n * sizeof(vg_digest), cudaMemcpyDeviceToDevice, c->stream));
-    if (n < sz) {
-        if (c->hash_kind == VG_HASH_SHA256)
-            k_fill_pad<VG_HASH_SHA256><<<grid_for(sz - n, HASH_THREADS), HASH_THREADS, 0, c->stream>>>((uint64_t *)tree, sz + n, 2 * sz);
-        else
-            k_fill_pad<VG_HASH_SHA3_256><<<grid_for(sz - n, HASH_THREADS), HASH_THREADS, 0, c->stream>>>((uint64_t *)tree, sz + n, 2 * sz);
-        VG_LAUNCHED(c);
+    TreeJobs j{};
+    j.t[0] = {(uint64_t *)tree, sz, n};
+    j.count = 1;
+    const uint64_t *pad = pad_table(c->hash_kind);
+    j.padded = n < sz;
+    memcpy(j.pad, pad, sizeof j.pad);
+    const vg_digest *src = leaves;
+    if (((uintptr_t)leaves & 15) || !vg_is_device_ptr(leaves)) {   // copied first; the kernel reads them in place
+        VG_CHECK_CUDA(cudaMemcpyAsync(tree + sz, leaves, n * sizeof(vg_digest), cudaMemcpyDeviceToDevice, c->stream));
+        src = tree + sz;
     }
-    return vg_merkle_build(c, (uint64_t *)tree, sz);
+    k_tree_leaves<<<std::min<unsigned>(grid_for(2 * sz, 256), 148u * 8u), 256, 0, c->stream>>>(
+        (const ulonglong2 *)src, n, sz, make_ulonglong2(pad[0], pad[1]), make_ulonglong2(pad[2], pad[3]), (ulonglong2 *)tree);
+    VG_LAUNCHED(c);
+    return vg_merkle_trees(c, j, nullptr);
 }
 
 extern "C" int vg_leaf_chain(vg_ctx *c, const vg_fe *cw, int n_slices, long n, vg_digest *leaves)

@@ -14,6 +14,7 @@ constexpr int MAX_HASH_JOBS = 16;
 // subtree of SUB_WIDTH parents and its levels above (vg_merkle_trees)
 constexpr long MERKLE_SUB_MAX = 8192;
 constexpr int SUB_WIDTH = 64, SUB_LEVELS = 7;
+constexpr int PAD_HEIGHTS = 24;   // of the levels above that, which reach 2^(13 + 24) leaves
 struct ChainJob {
     const fe *cw;       // slice-major codeword set, slices of n
     long n;
@@ -29,10 +30,13 @@ struct ChainJobs {
 struct TreeJob {
     uint64_t *tree;   // heap-ordered, leaves at [nleaves, 2 nleaves)
     long nleaves;     // power of two
+    long nreal;       // leaves before the padding (H(0^64), the last ones); nleaves when there is none
 };
 struct TreeJobs {
     TreeJob t[MAX_HASH_JOBS];
     int count;
+    bool padded;                      // some nreal < nleaves; then
+    uint64_t pad[4 * PAD_HEIGHTS];    // the digest of a subtree of 2^h padding leaves at 4 h
 };
 int vg_leaf_chains(vg_ctx *c, const ChainJobs &jobs);
 // Builds every tree; roots_dev (or null) receives 4 words per tree of at least two leaves, in job order.

@@ -77,9 +77,9 @@ static void sha256_64(const uint8_t *in, uint8_t *out)
     }
 }
 
-void virgo_hash64(const void *src, void *dst)
+void virgo_hash64_kind(int kind, const void *src, void *dst)
 {
-    if (virgo_hash_kind() == 1) {
+    if (kind == 1) {
         sha256_64((const uint8_t *)src, (uint8_t *)dst);
         return;
     }
@@ -88,3 +88,5 @@ void virgo_hash64(const void *src, void *dst)
     sha3_256_64(w, d);
     memcpy(dst, d, 32);
 }
+
+void virgo_hash64(const void *src, void *dst) { virgo_hash64_kind(virgo_hash_kind(), src, dst); }
