@@ -455,8 +455,8 @@ enum {
     VG_TUNE_BETA_TABLE = 8,    /* phase-2 table builds read each gate's beta_g from a table the
                                   phase-1 builds of the same layer wrote (1), or form it again
                                   from the eq half tables (0) */
-    VG_TUNE_GROUP_SPLIT = 9,   /* round groups: steps with few pairs left spread each pair over three
-                                  threads, one per table (1), or keep one thread per pair (0) */
+    VG_TUNE_GROUP_SPLIT = 9,   /* accepted, without effect: a round group's folds always take one thread
+                                  per table entry */
     VG_TUNE_LAZY_FOLD = 10,    /* accepted, without effect: the sumcheck folds x0 + r (x1 - x0) have
                                   one form, the unreduced difference and four products */
     VG_TUNE_GATHER_FUSE = 11,  /* deferred proofs with paired rounds: a phase's table build over

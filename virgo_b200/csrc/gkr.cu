@@ -675,32 +675,22 @@ __global__ void __launch_bounds__(GKR_THREADS) k_heavy_finish(HeavyKeys H, const
 // Round folds only combine neighbouring entries, so a CTA that owns a
 // contiguous chunk of the three tables can run several consecutive rounds on
 // it without any other CTA: a chunk of 2 RG_CHUNK entries folds into shared
-// memory (RG_CHUNK entries) and keeps folding there until two entries are
-// left, i.e. up to 10 rounds.  The challenges of all those rounds are known
-// in advance (they come from the verifier's rand() stream), so one launch
-// replaces up to 10 round launches and each table is read from HBM once per
-// group instead of once per round.  Per-round partial sums are reduced by
-// the last CTA to finish, which then runs the group's tail: the entries the
-// chunks left (at most 2 RG_CHUNK, written out by every CTA) fold on in its
-// shared memory for up to 10 more rounds, so the rounds of a phase below the
-// group start take one launch.  Every round's sums go to its record.
-constexpr int RG_LOG = 10, RG_CHUNK = 1 << RG_LOG, RG_THREADS = 256;
+// memory (RG_CHUNK entries) and keeps folding there.  The challenges of all
+// those rounds are known in advance (they come from the verifier's rand()
+// stream), so one launch replaces up to 10 round launches and each table is
+// read from HBM once per group instead of once per round.  The last CTA to
+// finish then runs the group's tail: the entries the chunks left (at most
+// 2 RG_CHUNK, written out by every CTA) fold on in its shared memory for up to
+// 10 more rounds, so the rounds of a phase below the group start take one
+// launch.  Every round's sums go to its record.
+constexpr int RG_LOG = 10, RG_CHUNK = 1 << RG_LOG, RG_THREADS = 512;
 // rounds of the chunks (RG_MAX) and of a whole launch with its tail (RG_STEPS)
 constexpr int RG_MAX = 12, RG_STEPS = 20;
-// Per-round partial sums of a group's CTAs ([round][CTA][3]): a group on
-// tables of up to N entries has at most N / RG_CHUNK CTAs, and a group split
-// into small chunks (at most 2 RG_CHUNK entries) at most 2 RG_CHUNK.
-static inline size_t rg_parts_len(long N) { return ((size_t)N / RG_CHUNK + 1 + 2 * RG_CHUNK) * RG_MAX * 3; }
-
-// shared-memory index of table entry i: one pad entry per 8 keeps the
-// stride-4 reads (entries 4k .. 4k+3 of a pair) and the stride-2 writes free
-// of bank conflicts
-__device__ __forceinline__ int rg_ix(long i) { return (int)(i + (i >> 3)); }
-constexpr int RG_TABLE = RG_CHUNK + RG_CHUNK / 8;
-// dynamic shared memory of a group CTA (elements): three tables, per-warp
-// round sums, each round's totals and challenge, the folded pairs of the
-// three-thread steps
-constexpr int RG_SMEM_FE = 3 * RG_TABLE + RG_STEPS * (RG_THREADS / 32) * 3 + RG_STEPS * 4 + 6 * (RG_THREADS / 3);
+constexpr int RG_LIMBS = 3 * LIMBS;        // limb sums of a round's three values
+constexpr int RG_LEVELS = 2 * RG_CHUNK;    // a table's folds of a job, all kept: 1024 + 512 + ... entries
+constexpr int RG_UNITS = 40;               // warps' worth of pairs in a job: 16 + 8 + 4 + 2 + 1 + 1 ...
+// dynamic shared memory of a group CTA
+constexpr int RG_SMEM = (3 * RG_LEVELS + RG_STEPS) * (int)sizeof(fe) + RG_STEPS * RG_LIMBS * 8 + RG_UNITS * RG_LIMBS * 4;
 struct RoundGroup {
     int chunk_log;      // log2 of a CTA's entries after its first step (at most RG_LOG)
     int nsteps;         // rounds in this launch, the tail's included (at most RG_STEPS)
@@ -708,7 +698,6 @@ struct RoundGroup {
     int first_nofold;   // the first round has no fold (the round right after a phase init)
     int slot0;          // record of the first round; the others follow
     int last6;          // write the final pair (the table ends at 2 entries) into the last record
-    int split3;         // steps with at most RG_THREADS / 3 pairs run three threads per pair
     const fe *r;        // fold challenge of each round (device memory, nsteps values)
 };
 
@@ -758,73 +747,34 @@ __device__ __forceinline__ void ld_rec3(fe (&x)[3], const fe *p)
     for (int k = 0; k < 3; ++k) x[k] = ld_fe_cg(p + k);
 }
 
-// warp sums of acc added into sm[step][warp][3] (a CTA's chunks accumulate
-// there); warps without an active lane (first thread >= active) add nothing
-__device__ __forceinline__ void rg_warp_add(fe (&acc)[3], fe *sm, int step, long active)
-{
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if ((long)(threadIdx.x & ~31) >= active) return;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) acc[k] = warp_sum(acc[k]);
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            fe *o = &sm[(step * (RG_THREADS / 32) + wid) * 3 + k];
-            *o = *o + acc[k];
-        }
-    }
-}
-
-// The x terms of a group's rounds after its first (rg_derive), in shared
-// memory:
-//   b_st = a_{st-1} r^2 + b_{st-1} r + c_{st-1} - 2 c_st - a_st.
-// The terms without b_{st-1} are formed
-// by one thread per round, then one thread runs the chain b_st = r b_{st-1}
-// + d_st.  tot: [round][3]; sr: the challenges; d: scratch [round].
-__device__ __forceinline__ void rg_derive_smem(fe *tot, const fe *sr, fe *d, int nsteps)
-{
-    const int t = threadIdx.x;
-    if (t >= 1 && t < nsteps) {
-        const fe r = sr[t];
-        const fe *p = tot + 3 * (t - 1), *o = tot + 3 * t;
-        d[t] = ((p[0] * (r * r) + p[2]) - (o[2] + o[2])) - o[0];
-    }
-    __syncthreads();
-    if (t == 0) {
-        fe b = tot[1];
-        for (int st = 1; st < nsteps; ++st) {
-            b = sr[st] * b + d[st];
-            tot[3 * st + 1] = b;
-        }
-    }
-    __syncthreads();
-}
-
 // CTAs loop over the chunks (chunk q at q * cin of the input), so the grid
-// stays within what is resident at once and the last CTA's reduction reads
-// at most gridDim.x partials per round.  Each CTA runs its chunks as jobs,
-// and the last one then runs the tail as one more job through the same step
-// code (one copy of it: the default kernel stays small enough for the
-// instruction cache).  The tail reads the chunks' remaining entries at L2,
-// after the fence and counter that order every CTA's writes before it.
-// SPLIT: the three-thread steps (VG_TUNE_GROUP_SPLIT) are compiled in only
-// when asked for, for the same reason
-template <bool SPLIT>
+// stays within what is resident at once.  Each CTA runs its chunks as jobs,
+// and the last one then runs the tail as one more job through the same code
+// (one copy of it: the kernel stays small enough for the instruction cache).
+//
+// A job is bound by latency: its rounds depend on one another only through
+// the folds.  So the folds run first, one entry per thread and a barrier per
+// level (the last levels, at most 32 entries, in one warp without barriers),
+// every level kept in shared memory; then all rounds' sums are formed at once,
+// a warp's worth of pairs after another with no waiting between rounds, and
+// reduced as limbs (warp_limbs).  All three sums are formed (the x term from
+// the values at 1), which costs a product per pair and saves the chain of
+// claims.  Folding and summing round by round, with two barriers and a tree of
+// field additions each, took 35 us for the 16 rounds of a 2^17-entry table;
+// the side proof of 2^11 (24 groups) went from 1.2 to 0.54 ms.
 __global__ void __launch_bounds__(RG_THREADS) k_round_group(const fe *__restrict__ xV, const fe *__restrict__ xA,
                                                             const fe *__restrict__ xM, long n_in, RoundGroup G,
-                                                            fe *yV, fe *yA, fe *yM, fe *__restrict__ parts,
+                                                            fe *yV, fe *yA, fe *yM, unsigned long long *__restrict__ gacc,
                                                             unsigned *__restrict__ counter, fe *__restrict__ rec)
 {
     extern __shared__ fe smem[];
     constexpr int NW = RG_THREADS / 32;
-    fe *sV = smem, *sA = smem + RG_TABLE, *sM = smem + 2 * RG_TABLE;
-    fe *wsum = smem + 3 * RG_TABLE;        // [RG_STEPS][warps][3]
-    fe *tot = wsum + RG_STEPS * NW * 3;    // [RG_STEPS][3]: each round's sums over the whole table
-    fe *sr = tot + RG_STEPS * 3;           // [RG_STEPS]: the rounds' challenges
-    fe *stage = sr + RG_STEPS;             // [pair][6] of the three-thread steps; the epilogue's scratch
+    fe *tab = smem;                                    // [3][RG_LEVELS]: V, addV, add_mult, level after level
+    fe *sr = tab + 3 * RG_LEVELS;                      // [RG_STEPS]: the rounds' challenges
+    unsigned long long *lim = reinterpret_cast<unsigned long long *>(sr + RG_STEPS);   // [RG_STEPS][RG_LIMBS]
+    uint32_t *us = reinterpret_cast<uint32_t *>(lim + RG_STEPS * RG_LIMBS);            // [RG_UNITS][RG_LIMBS]
     __shared__ bool last;
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-    for (int i = t; i < RG_STEPS * NW * 3; i += RG_THREADS) wsum[i] = vg::fe_zero();
     if (t < G.nsteps) sr[t] = ld_fe_cg(G.r + t);
     const int k1 = G.nsteps - G.tail;      // rounds of the chunks
     const long chunk = 1L << G.chunk_log;
@@ -832,179 +782,157 @@ __global__ void __launch_bounds__(RG_THREADS) k_round_group(const fe *__restrict
     const long nchunks = n_in / cin;
     const long mfin = (G.first_nofold ? cin : cin / 2) >> (k1 - 1);   // entries a chunk leaves
     const bool alone = gridDim.x == 1;
-    long m = 0;          // entries in shared memory
-    bool tail = false;   // the job is the tail (after every chunk)
+    unsigned long long acc = 0;   // thread t: limb t % RG_LIMBS of round t / RG_LIMBS of the jobs so far
+    bool tail = false;            // the job is the tail (after every chunk)
     for (long q = blockIdx.x;;) {
         if (!tail && q >= nchunks) {
             // every chunk of this CTA is done: its round sums
-            __syncthreads();
             if (alone) {   // a single CTA: its sums are the totals
-                if (t < 3 * k1) {
-                    fe x = vg::fe_zero();
-                    for (int w = 0; w < NW; ++w) x = x + wsum[((t / 3) * NW + w) * 3 + t % 3];
-                    tot[t] = x;
-                }
+                if (t < RG_LIMBS * k1) lim[t] = acc;
             } else {
-                if (t < 3 * k1) {
-                    fe x = vg::fe_zero();
-                    for (int w = 0; w < NW; ++w) x = x + wsum[((t / 3) * NW + w) * 3 + t % 3];
-                    parts[((long)(t / 3) * gridDim.x + blockIdx.x) * 3 + t % 3] = x;
-                }
+                if (t < RG_LIMBS * k1) atomicAdd(&gacc[t], acc);
                 __threadfence();
                 __syncthreads();
                 if (t == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
                 __syncthreads();
                 if (!last) return;
                 __threadfence();
-                // warp st sums round st over all CTAs, four partials in flight per lane
-                for (int st = wid; st < k1; st += NW) {
-                    fe s3[3] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
-                    for (long b0 = lane; b0 < gridDim.x; b0 += 4 * 32) {
-                        fe x[4][3];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const long b = b0 + 32 * j;
-#pragma unroll
-                            for (int k = 0; k < 3; ++k)
-                                x[j][k] = b < gridDim.x ? ld_fe_cg(&parts[((long)st * gridDim.x + b) * 3 + k])
-                                                        : vg::fe_zero();
-                        }
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-#pragma unroll
-                            for (int k = 0; k < 3; ++k) s3[k] = s3[k] + x[j][k];
-                    }
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) s3[k] = warp_sum(s3[k]);
-                    if (lane == 0) {
-                        tot[3 * st] = s3[0];
-                        tot[3 * st + 1] = s3[1];
-                        tot[3 * st + 2] = s3[2];
-                    }
+                if (t < RG_LIMBS * k1) {
+                    lim[t] = __ldcg(&gacc[t]);
+                    gacc[t] = 0;
                 }
+                if (t == 0) *counter = 0;
             }
+            acc = 0;
             if (!G.tail) break;
             tail = true;
         }
         // one job: chunk q (rounds 0 .. k1-1), or the tail (rounds k1 .. nsteps-1)
         const fe *X0 = tail ? yV : xV, *X1 = tail ? yA : xA, *X2 = tail ? yM : xM;
-        const long base = tail ? 0 : q * cin, nin = tail ? nchunks * mfin : cin;
+        const long base = tail ? 0 : q * cin;
+        const int nin = (int)(tail ? nchunks * mfin : cin);
         const bool nofold = !tail && G.first_nofold;
-        const int st0 = tail ? k1 : 0, st1 = tail ? G.nsteps : k1;
-        m = nofold ? nin : nin / 2;   // entries in shared memory after the first step
-        __syncthreads();   // wsum zeroed, sr loaded; the previous job's tables written out
-        // first step: from global into shared
-        {
-            fe acc[3] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
+        const int st0 = tail ? k1 : 0, nr = (tail ? G.nsteps : k1) - st0;
+        const int m0 = nofold ? nin : nin / 2, lg0 = 31 - __clz(m0);   // entries of the first level
+        __syncthreads();   // sr loaded; the previous job's levels and unit sums read
+        {   // first level: from global into shared
             const vg::fold_r r = vg::fold_prep(sr[st0]);
-            for (long k = t; k < m / 2; k += RG_THREADS) {
-                fe v0, v1, a0, a1, m0v, m1v;
-                if (nofold) {
-                    const long b = base + 2 * k;
-                    v0 = ld_fe_cg(X0 + b); v1 = ld_fe_cg(X0 + b + 1);
-                    a0 = ld_fe_cg(X1 + b); a1 = ld_fe_cg(X1 + b + 1);
-                    m0v = ld_fe_cg(X2 + b); m1v = ld_fe_cg(X2 + b + 1);
-                } else {
-                    const long b = base + 4 * k;
-                    v0 = vg::fe_fold(ld_fe_cg(X0 + b), ld_fe_cg(X0 + b + 1), r);
-                    v1 = vg::fe_fold(ld_fe_cg(X0 + b + 2), ld_fe_cg(X0 + b + 3), r);
-                    a0 = vg::fe_fold(ld_fe_cg(X1 + b), ld_fe_cg(X1 + b + 1), r);
-                    a1 = vg::fe_fold(ld_fe_cg(X1 + b + 2), ld_fe_cg(X1 + b + 3), r);
-                    m0v = vg::fe_fold(ld_fe_cg(X2 + b), ld_fe_cg(X2 + b + 1), r);
-                    m1v = vg::fe_fold(ld_fe_cg(X2 + b + 2), ld_fe_cg(X2 + b + 3), r);
-                }
-                const int i0 = rg_ix(2 * k), i1 = rg_ix(2 * k + 1);
-                sV[i0] = v0; sV[i1] = v1;
-                sA[i0] = a0; sA[i1] = a1;
-                sM[i0] = m0v; sM[i1] = m1v;
-                rg_sums(v0, v1, a0, a1, m0v, m1v, acc);
+#pragma unroll 4
+            for (int i = t; i < 3 * m0; i += RG_THREADS) {
+                const int w = i >> lg0, k = i & (m0 - 1);
+                const fe *X = (w == 0 ? X0 : (w == 1 ? X1 : X2)) + base;
+                tab[w * RG_LEVELS + k] = nofold ? ld_fe_cg(X + k)
+                                                : vg::fe_fold(ld_fe_cg(X + 2 * k), ld_fe_cg(X + 2 * k + 1), r);
             }
-            rg_sums_end(acc);
-            rg_warp_add(acc, wsum, st0, m / 2);
-        }
-        // further steps in shared memory: fold m -> m/2, sums over m/4 pairs
-        for (int st = st0 + 1; st < st1; ++st) {
-            const vg::fold_r r = vg::fold_prep(sr[st]);
-            const long npairs = m / 4;
-            if (SPLIT && 3 * npairs <= RG_THREADS) {
-                // few pairs: three threads per pair, one per table, each
-                // folding its table's two entries; the folded pairs meet in
-                // `stage`, and the V and add_mult threads add the x^0 and x^2
-                // sums (p0 = m0 v0 plus a0, p2 = (m1 - m0)(v1 - v0)); the x
-                // term follows from the claim (rg_derive_smem)
-                const int pp = t / 3, role = t - 3 * pp;
-                const bool act = pp < npairs;
-                fe *tab = role == 0 ? sV : (role == 1 ? sA : sM);
-                fe f0 = vg::fe_zero(), f1 = vg::fe_zero();
-                __syncthreads();
-                if (act) {
-                    f0 = vg::fe_fold(tab[rg_ix(4 * pp)], tab[rg_ix(4 * pp + 1)], r);
-                    f1 = vg::fe_fold(tab[rg_ix(4 * pp + 2)], tab[rg_ix(4 * pp + 3)], r);
-                    stage[6 * pp + 2 * role] = f0;
-                    stage[6 * pp + 2 * role + 1] = f1;
-                }
-                __syncthreads();   // every read of this step's tables is done
-                fe acc[3] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
-                if (act) {
-                    tab[rg_ix(2 * pp)] = f0;
-                    tab[rg_ix(2 * pp + 1)] = f1;
-                    const fe *s6 = stage + 6 * pp;   // v0 v1 a0 a1 m0 m1
-                    if (role == 0) acc[2] = s6[4] * s6[0] + s6[2];
-                    else if (role == 2) acc[0] = (s6[5] - s6[4]) * (s6[1] - s6[0]);
-                }
-                m >>= 1;
-                rg_warp_add(acc, wsum, st, 3 * npairs);
-                continue;
-            }
-            fe acc[3] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
-            fe v0, v1, a0, a1, m0v, m1v;
-            __syncthreads();
-            const bool act = t < npairs;   // m / 4 <= RG_CHUNK / 4 = RG_THREADS: at most one pair per thread
-            if (act) {
-                const int b0 = rg_ix(4 * t), b1 = rg_ix(4 * t + 1), b2 = rg_ix(4 * t + 2), b3 = rg_ix(4 * t + 3);
-                v0 = vg::fe_fold(sV[b0], sV[b1], r); v1 = vg::fe_fold(sV[b2], sV[b3], r);
-                a0 = vg::fe_fold(sA[b0], sA[b1], r); a1 = vg::fe_fold(sA[b2], sA[b3], r);
-                m0v = vg::fe_fold(sM[b0], sM[b1], r); m1v = vg::fe_fold(sM[b2], sM[b3], r);
-                rg_sums<false>(v0, v1, a0, a1, m0v, m1v, acc);
-            }
-            __syncthreads();
-            if (act) {
-                const int i0 = rg_ix(2 * t), i1 = rg_ix(2 * t + 1);
-                sV[i0] = v0; sV[i1] = v1;
-                sA[i0] = a0; sA[i1] = a1;
-                sM[i0] = m0v; sM[i1] = m1v;
-            }
-            m >>= 1;
-            rg_warp_add(acc, wsum, st, npairs);
         }
         __syncthreads();
-        // the job's remaining m entries (none when the group folded nothing);
-        // the tail's go to the start of the same tables, every read of them done
-        const long yo = tail ? 0 : q * m;
-        for (long k = t; yV && k < m; k += RG_THREADS) {
-            yV[yo + k] = sV[rg_ix(k)];
-            yA[yo + k] = sA[rg_ix(k)];
-            yM[yo + k] = sM[rg_ix(k)];
+        // further levels in shared memory, m -> m / 2
+        int off = 0, m = m0, lg = lg0, lv = 0;
+        auto level = [&](int i0, int stride) {
+            const vg::fold_r r = vg::fold_prep(sr[st0 + lv + 1]);
+            const int mn = m >> 1;
+            for (int i = i0; i < 3 * mn; i += stride) {
+                const int w = i >> (lg - 1), k = i & (mn - 1);
+                fe *T = tab + w * RG_LEVELS + off;
+                T[m + k] = vg::fe_fold(T[2 * k], T[2 * k + 1], r);
+            }
+            off += m;
+            m = mn;
+            --lg;
+            ++lv;
+        };
+        while (lv + 1 < nr && 3 * (m >> 1) > 32) {
+            level(t, RG_THREADS);
+            __syncthreads();
         }
+        const int lc = lv;   // levels 0 .. lc are complete; warp 0 folds the others, the other warps go on
+        if (wid == 0) {
+            while (lv + 1 < nr) {
+                level(lane, 32);
+                __syncwarp();
+            }
+        }
+        // the rounds' sums: units of 32 pairs of a level, those of levels
+        // 0 .. lc over the warps (without warp 0 while it folds), the last levels' in warp 0
+        {
+            const int w0 = lc + 1 < nr ? 1 : 0;
+            int unit = 0, mine = wid - w0, o = 0;
+            for (int l = 0; l < nr; ++l) {
+                const int ml = m0 >> l, pairs = ml >> 1, nu = max(1, pairs >> 5);
+                for (int u = 0; u < nu; ++u, ++unit) {
+                    bool take;
+                    if (l <= lc) {
+                        take = mine == 0;
+                        mine = mine <= 0 ? (mine < 0 ? mine : NW - w0 - 1) : mine - 1;
+                    } else {
+                        take = wid == 0;
+                    }
+                    if (!take) continue;
+                    const int k = 32 * u + lane;
+                    fe A = vg::fe_zero(), C = A, E = A;
+                    if (k < pairs) {
+                        const fe *T = tab + o + 2 * k;
+                        const fe v0 = T[0], v1 = T[1], a0 = T[RG_LEVELS], a1 = T[RG_LEVELS + 1], x0 = T[2 * RG_LEVELS],
+                                 x1 = T[2 * RG_LEVELS + 1];
+                        A = vg::fe_fma_diff(A, x1 - x0, v0, v1);
+                        C = vg::fe_fma(a0, x0, v0);
+                        E = vg::fe_fma(a1, x1, v1);
+                    }
+                    uint32_t lA[LIMBS], lC[LIMBS], lE[LIMBS];
+                    warp_limbs(A, lA);
+                    warp_limbs(C, lC);
+                    warp_limbs(E, lE);
+                    if (lane == 0) {
+                        uint32_t *d = us + unit * RG_LIMBS;
+#pragma unroll
+                        for (int j = 0; j < LIMBS; ++j) {
+                            d[j] = lA[j];
+                            d[LIMBS + j] = lE[j];
+                            d[2 * LIMBS + j] = lC[j];
+                        }
+                    }
+                }
+                o += ml;
+            }
+        }
+        __syncthreads();
+        if (t < RG_LIMBS * nr) {   // nr <= RG_MAX: at most 216 threads
+            const int l = t / RG_LIMBS, j = t - l * RG_LIMBS;
+            int u0 = 0;
+            for (int i = 0; i < l; ++i) u0 += max(1, m0 >> (i + 1) >> 5);
+            const int nu = max(1, m0 >> (l + 1) >> 5);
+            for (int u = 0; u < nu; ++u) acc += us[(u0 + u) * RG_LIMBS + j];
+            if (tail) lim[RG_LIMBS * k1 + t] = acc;
+        }
+        // the job's remaining entries (none when the group folded nothing);
+        // the tail's go to the start of the same tables, every read of them done
+        const int mlast = m0 >> (nr - 1), olast = 2 * (m0 - mlast);
+        const long yo = tail ? 0 : q * mlast;
+        for (int k = t; yV && k < mlast; k += RG_THREADS) {
+            yV[yo + k] = tab[olast + k];
+            yA[yo + k] = tab[RG_LEVELS + olast + k];
+            yM[yo + k] = tab[2 * RG_LEVELS + olast + k];
+        }
+        if (G.last6 && mlast == 2 && t < 6 && (tail || !G.tail))
+            rec[9 * (G.slot0 + G.nsteps - 1) + 3 + t] = tab[(t >> 1) * RG_LEVELS + olast + (t & 1)];
         if (tail) break;
         q += gridDim.x;
     }
-    // a single CTA or the last one: the tail's sums (its own warps'), the
-    // final pair, the x terms, the records
+    // a single CTA or the last one: the records
     __syncthreads();
-    if (tail && t < 3 * G.tail) {
-        fe x = vg::fe_zero();
-        for (int w = 0; w < NW; ++w) x = x + wsum[((k1 + t / 3) * NW + w) * 3 + t % 3];
-        tot[3 * k1 + t] = x;
+    if (t < G.nsteps) {
+        fe x[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const unsigned long long *p = lim + t * RG_LIMBS + k * LIMBS;
+            x[k] = fe_from_limbs(p[0], p[1], p[2], p[3], p[4], p[5]);
+        }
+        rg_sums_end(x);
+        fe *o = rec + 9 * (G.slot0 + t);
+        o[0] = x[0];
+        o[1] = x[1];
+        o[2] = x[2];
     }
-    if (G.last6 && m == 2 && t == 0) {
-        fe *l6 = rec + 9 * (G.slot0 + G.nsteps - 1) + 3;
-        l6[0] = sV[0]; l6[1] = sV[1]; l6[2] = sA[0]; l6[3] = sA[1]; l6[4] = sM[0]; l6[5] = sM[1];   // rg_ix(0, 1) = 0, 1
-    }
-    __syncthreads();
-    rg_derive_smem(tot, sr, stage, G.nsteps);
-    for (int i = t; i < 3 * G.nsteps; i += RG_THREADS) rec[9 * (G.slot0 + i / 3) + i % 3] = tot[i];
-    if (!alone && t == 0) *counter = 0;
 }
 
 // ------------------------------------------------ verifier's wiring predicates
@@ -1506,7 +1434,7 @@ struct vg_gkr {
     long pend_n0 = 0;                    // table length before the group's first round
     long pend_chunk = 0;                 // a CTA's entries after its first step
     bool pend_nofold = false;
-    fe *rg_parts = nullptr;              // per-CTA, per-round partial sums of a group
+    unsigned long long *rg_acc = nullptr;   // a group's limb sums over its CTAs, zero between launches
     // deferred round above the group start held back to run together with
     // the next round in one k_round2 pass (VG_TUNE_ROUND_FUSE = 2)
     bool held = false;
@@ -2009,16 +1937,13 @@ static int gkr_bind(vg_gkr *g, const vg_circuit *c)
                 g->buf[b][k] = nullptr;
             }
         vg_release(x, g->eq);
-        vg_release(x, g->rg_parts);
         vg_release(x, g->bgt);
-        g->eq = g->rg_parts = g->bgt = nullptr;
+        g->eq = g->bgt = nullptr;
         g->N_cap = 0;
         for (int b = 0; b < 2; ++b)
             for (int k = 0; k < 3; ++k)
                 if (vg_alloc(x, (void **)&g->buf[b][k], (b == 0 ? N : N / 2 + 1) * sizeof(fe)) != VG_OK) return oom("tables");
         if (vg_alloc(x, (void **)&g->eq, 6 * (1L << (c->max_bl / 2 + 1)) * sizeof(fe)) != VG_OK) return oom("eq tables");
-        if (vg_alloc(x, (void **)&g->rg_parts, rg_parts_len(N) * sizeof(fe)) != VG_OK)
-            return oom("group partials");
         if (vg_alloc(x, (void **)&g->bgt, N * sizeof(fe)) != VG_OK) return oom("beta_g table");
         g->N_cap = N;
     }
@@ -2057,6 +1982,7 @@ extern "C" int vg_gkr_create(vg_ctx *ctx, const vg_circuit *c, vg_gkr **out)
     };
     if (cudaMalloc(&g->rbuf, 3 * 64 * sizeof(fe)) != cudaSuccess) return fail("challenges");
     if (cudaMalloc(&g->round_acc, LIMBS * 6 * 8) != cudaSuccess) return fail("round sums");
+    if (cudaMalloc(&g->rg_acc, RG_MAX * RG_LIMBS * 8) != cudaSuccess) return fail("group sums");
     if (cudaMalloc(&g->round_out, 16 * sizeof(fe)) != cudaSuccess) return fail("round sums");
     if (cudaMalloc(&g->round_counter, sizeof(unsigned)) != cudaSuccess) return fail("round counter");
     if (cudaMalloc(&g->vu, sizeof(fe)) != cudaSuccess) return fail("v_u");
@@ -2067,7 +1993,8 @@ extern "C" int vg_gkr_create(vg_ctx *ctx, const vg_circuit *c, vg_gkr **out)
     // on the context's stream: the streams are non-blocking, so a memset on
     // the legacy stream would not be ordered before the first round kernel
     if (cudaMemsetAsync(g->round_counter, 0, sizeof(unsigned), ctx->stream) != cudaSuccess ||
-        cudaMemsetAsync(g->round_acc, 0, LIMBS * 6 * 8, ctx->stream) != cudaSuccess)
+        cudaMemsetAsync(g->round_acc, 0, LIMBS * 6 * 8, ctx->stream) != cudaSuccess ||
+        cudaMemsetAsync(g->rg_acc, 0, RG_MAX * RG_LIMBS * 8, ctx->stream) != cudaSuccess)
         return fail("round counter");
     int rc = gkr_bind(g, c);
     if (rc != VG_OK) {
@@ -2100,7 +2027,7 @@ extern "C" int vg_gkr_destroy(vg_gkr *g)
     cudaFree(g->round_counter);
     cudaFree(g->vu);
     cudaFree(g->heavy_parts);
-    cudaFree(g->rg_parts);
+    cudaFree(g->rg_acc);
     cudaFree(g->bgt);
     cudaFree(g->rec);
     if (g->rec_host) cudaFreeHost(g->rec_host);
@@ -2518,6 +2445,12 @@ static bool fuse_gather(vg_gkr *g, long N)
            N > S && N >= 8;
 }
 
+// Entries a CTA of a group on a table of n0 entries holds after its first
+// fold: short chunks on many CTAs (their rounds are latency), as long as the
+// last CTA's tail stays within one CTA.
+// 2^17 entries run as 128 CTAs of 1024, not 64 of 2048.
+static long group_chunk(long n0) { return std::max(64L, std::min((long)RG_CHUNK, n0 / 256)); }
+
 // Rounds the chunks of a group starting at table length n0 with chunks of
 // `chunk` can hold (see k_round_group).
 static int group_capacity(long n0, bool nofold, long chunk)
@@ -2567,9 +2500,7 @@ static int rg_smem_attribute(int dev)
     std::lock_guard<std::mutex> lock(mu);
     if (dev >= (int)done.size()) done.resize(dev + 1, false);
     if (!done[dev]) {
-        const int bytes = (int)(RG_SMEM_FE * sizeof(fe));
-        VG_CHECK_CUDA(cudaFuncSetAttribute(k_round_group<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        VG_CHECK_CUDA(cudaFuncSetAttribute(k_round_group<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        VG_CHECK_CUDA(cudaFuncSetAttribute(k_round_group, cudaFuncAttributeMaxDynamicSharedMemorySize, RG_SMEM));
         done[dev] = true;
     }
     return VG_OK;
@@ -2623,12 +2554,8 @@ static int issue_launch(vg_gkr *g, const RoundLaunch &L, const fe *rp)
         } else {
             RoundGroup G = L.G;
             G.r = rp;
-#define VG_GROUP_LAUNCH(SP)                                                                                          \
-    k_round_group<SP><<<L.grid, RG_THREADS, RG_SMEM_FE * sizeof(fe), c->stream>>>(                                   \
-        L.x[0], L.x[1], L.x[2], L.count, G, L.y[0], L.y[1], L.y[2], g->rg_parts, g->round_counter, g->rec)
-            if (G.split3) VG_GROUP_LAUNCH(true);
-            else VG_GROUP_LAUNCH(false);
-#undef VG_GROUP_LAUNCH
+            k_round_group<<<L.grid, RG_THREADS, RG_SMEM, c->stream>>>(L.x[0], L.x[1], L.x[2], L.count, G, L.y[0], L.y[1],
+                                                                      L.y[2], g->rg_acc, g->round_counter, g->rec);
         }
     }
     VG_LAUNCHED(c);
@@ -2718,8 +2645,7 @@ static int exec_pending(vg_gkr *g)
         key.push_back((uint64_t)(uintptr_t)L.ob);
         key.push_back((uint64_t)(uintptr_t)L.prev);
         key.push_back(((uint64_t)L.G.chunk_log) | ((uint64_t)L.G.nsteps << 8) | ((uint64_t)L.G.first_nofold << 16) |
-                      ((uint64_t)L.G.last6 << 24) | ((uint64_t)L.G.split3 << 32) |
-                      ((uint64_t)L.G.tail << 40));
+                      ((uint64_t)L.G.last6 << 24) | ((uint64_t)L.G.tail << 40));
         key.push_back((uint64_t)L.G.slot0);
         if (L.kind == 3) {
             const GatherArgs &a = L.ga;
@@ -2733,7 +2659,7 @@ static int exec_pending(vg_gkr *g)
     }
     key.push_back((uint64_t)(uintptr_t)g->round_acc);
     key.push_back((uint64_t)(uintptr_t)g->round_counter);
-    key.push_back((uint64_t)(uintptr_t)g->rg_parts);
+    key.push_back((uint64_t)(uintptr_t)g->rg_acc);
     key.push_back((uint64_t)(uintptr_t)g->rec);
     uint64_t h = 1469598103934665603ull;   // FNV-1a over the key words
     for (uint64_t w : key) {
@@ -2886,10 +2812,9 @@ static int group_rounds(vg_gkr *g)
         return vg_fail(VG_ERR_STATE, "round group of %d rounds on %ld entries", G.nsteps, n_in);
     G.tail = gs.tail;
     const long nchunks = gs.nchunks;
-    // CTAs loop over chunks: at most 3 resident per SM (72 KB of shared memory each)
-    L.grid = (unsigned)std::min(nchunks, 148L * 3L);
+    // CTAs loop over chunks: at most 2 resident per SM (101 KB of shared memory each)
+    L.grid = (unsigned)std::min(nchunks, 148L * 2L);
     G.last6 = (gs.final_n == 2 && (gs.tail || nchunks == 1)) ? 1 : 0;
-    G.split3 = vg_tune_value(c->device, VG_TUNE_GROUP_SPLIT) != 0 ? 1 : 0;
     const bool folds = !(G.first_nofold && G.nsteps == 1);
     L.threads = RG_THREADS;
     L.count = n_in;
@@ -3066,7 +2991,7 @@ extern "C" int vg_gkr_round(vg_gkr *g, vg_fe previous_random, int current_bit, v
             g->pend_n0 = g->n;
             g->pend_nofold = !fold;
             g->pend_slot0 = g->rec_n;
-            g->pend_chunk = RG_CHUNK;
+            g->pend_chunk = group_chunk(g->n);
         }
         g->pend_r.push_back(tofe(previous_random));
         ++g->rec_n;
@@ -3142,11 +3067,13 @@ int vg_gkr_tables_create(vg_ctx *ctx, long max_n, int max_records, vg_gkr **out)
         return vg_fail(VG_ERR_OOM, "vg_gkr_tables_create: %s allocation failed", what);
     };
     if (cudaMalloc(&g->round_acc, LIMBS * 6 * 8) != cudaSuccess) return fail("round sums");
+    if (cudaMalloc(&g->rg_acc, RG_MAX * RG_LIMBS * 8) != cudaSuccess) return fail("group sums");
     if (cudaMalloc(&g->round_out, 16 * sizeof(fe)) != cudaSuccess) return fail("round sums");
     if (cudaMalloc(&g->round_counter, sizeof(unsigned)) != cudaSuccess) return fail("round counter");
     // ordered on the context's (non-blocking) stream before the first round
     if (cudaMemsetAsync(g->round_counter, 0, sizeof(unsigned), ctx->stream) != cudaSuccess ||
-        cudaMemsetAsync(g->round_acc, 0, LIMBS * 6 * 8, ctx->stream) != cudaSuccess)
+        cudaMemsetAsync(g->round_acc, 0, LIMBS * 6 * 8, ctx->stream) != cudaSuccess ||
+        cudaMemsetAsync(g->rg_acc, 0, RG_MAX * RG_LIMBS * 8, ctx->stream) != cudaSuccess)
         return fail("round counter");
     g->deferred = true;
     const int rc = vg_gkr_tables_reserve(g, max_n, max_records);
@@ -3173,13 +3100,10 @@ int vg_gkr_tables_reserve(vg_gkr *g, long max_n, int max_records)
                 vg_release(x, g->buf[b][k]);
                 g->buf[b][k] = nullptr;
             }
-        vg_release(x, g->rg_parts);
-        g->rg_parts = nullptr;
         g->N_cap = 0;
         for (int b = 0; b < 2; ++b)
             for (int k = 0; k < 3; ++k)
                 VG_TRY(vg_alloc(x, (void **)&g->buf[b][k], (b == 0 ? max_n : max_n / 2 + 1) * sizeof(fe)));
-        VG_TRY(vg_alloc(x, (void **)&g->rg_parts, rg_parts_len(max_n) * sizeof(fe)));
         g->N_cap = max_n;
     }
     if (max_records > g->rec_cap) {
