@@ -214,6 +214,10 @@ struct vg_pc {
     std::vector<PcLevel> levels;
     int nlevels = 0;
     bool have_private = false, have_public = false;
+    // the context of a whole commitment's second stream (vg_pc_prove_deferred):
+    // lent (vg_pc_set_side) or made on first use
+    vg_ctx *side = nullptr;
+    bool own_side = false;
     fe *F(DevBuf &b) { return (fe *)b.p; }
     uint64_t *U(DevBuf &b) { return (uint64_t *)b.p; }
 };
@@ -281,6 +285,7 @@ extern "C" int vg_pc_destroy(vg_pc *pc)
     if (!pc) return VG_OK;
     cudaStreamSynchronize(pc->ctx->stream);
     pc_free(pc);
+    if (pc->own_side) vg_ctx_destroy(pc->side);
     delete pc;
     return VG_OK;
 }
@@ -307,27 +312,32 @@ static int device_input(vg_pc *pc, const vg_fe *x, long N, const fe **out)
     return VG_OK;
 }
 
-// zero-padded mask of M entries on the device (poly_commit.h:66-70, 138-139);
-// with staging == nullptr through the context's pinned buffer (synchronised,
-// it is reused), else through the caller's pinned staging (not synchronised)
-static int device_mask(vg_pc *pc, DevBuf &dst, const vg_fe *mask, long n_mask, long M, fe *staging = nullptr)
+// zero-padded mask of M entries on the device (poly_commit.h:66-70, 138-139)
+// through the context's pinned buffer (synchronised, it is reused)
+static int device_mask(vg_pc *pc, DevBuf &dst, const vg_fe *mask, long n_mask, long M)
 {
     vg_ctx *c = pc->ctx;
     VG_TRY(ensure(c, dst, M * sizeof(fe)));
-    fe *host = staging;
-    if (!host) VG_TRY(vg_pinned(c, M, &host));
+    fe *host;
+    VG_TRY(vg_pinned(c, M, &host));
     for (long i = 0; i < M; ++i) host[i] = i < n_mask ? vg::fe_make(mask[i].real, mask[i].img) : vg::fe_zero();
     VG_CHECK_CUDA(cudaMemcpyAsync(dst.p, host, M * sizeof(fe), cudaMemcpyHostToDevice, c->stream));
-    if (!staging) VG_CHECK_CUDA(cudaStreamSynchronize(c->stream));
+    VG_CHECK_CUDA(cudaStreamSynchronize(c->stream));
+    return VG_OK;
+}
+// the same on context x through the caller's pinned staging (not synchronised)
+static int stage_mask(vg_ctx *x, DevBuf &dst, const vg_fe *mask, long n_mask, long M, fe *staging)
+{
+    for (long i = 0; i < M; ++i) staging[i] = i < n_mask ? vg::fe_make(mask[i].real, mask[i].img) : vg::fe_zero();
+    VG_CHECK_CUDA(cudaMemcpyAsync(dst.p, staging, M * sizeof(fe), cudaMemcpyHostToDevice, x->stream));
     return VG_OK;
 }
 
-static int encode_private(vg_pc *pc, const vg_fe *priv, int log_len, const vg_fe *mask, long n_mask, long *mask_len,
-                          fe *staging)
+// checks and sizes of a commitment to 2^log_len values with n_mask mask entries
+static int start_private(vg_pc *pc, const vg_fe *priv, int log_len, const vg_fe *mask, long n_mask)
 {
     if (!pc || !priv || !mask || n_mask < 1 || log_len < 7 || log_len > 28)
         return vg_fail(VG_ERR_ARG, "vg_pc_encode_private: bad argument (log_len=%d n_mask=%ld)", log_len, n_mask);
-    vg_ctx *c = pc->ctx;
     pc->have_private = pc->have_public = false;
     pc->nlevels = 0;
     pc->log_len = log_len;
@@ -336,16 +346,35 @@ static int encode_private(vg_pc *pc, const vg_fe *priv, int log_len, const vg_fe
     if (n_mask > pc->S) return vg_fail(VG_ERR_ARG, "mask longer than a slice (%ld > %ld)", n_mask, pc->S);
     pc->gap = mask_gap(pc->S, n_mask);
     pc->M = pc->S / pc->gap;
-    const long S = pc->S, R = pc->R, M = pc->M, N = 1L << log_len;
-    VG_TRY(ensure(c, pc->l_eval, 65 * S * sizeof(fe)));
-    const fe *priv_d;
-    VG_TRY(device_input(pc, priv, N, &priv_d));
+    return ensure(pc->ctx, pc->l_eval, 65 * pc->S * sizeof(fe));
+}
+
+// the data slices of l or q (out) from 2^log_len values
+static int encode_data(vg_pc *pc, const vg_fe *vals, fe *out)
+{
+    vg_ctx *c = pc->ctx;
+    const fe *d;
+    VG_TRY(device_input(pc, vals, 1L << pc->log_len, &d));
     fe *coef;
-    VG_TRY(vg_scratch2(c, 64 * R * sizeof(fe), (void **)&coef));
-    VG_TRY(rs_encode(c, priv_d, R, 64, pc->F(pc->l_eval), S, coef));
-    VG_TRY(device_mask(pc, pc->mask, mask, n_mask, M, staging));
-    VG_TRY(rs_encode(c, pc->F(pc->mask), M, 1, pc->F(pc->l_eval) + 64 * S, S, coef));
-    if (mask_len) *mask_len = M;
+    VG_TRY(vg_scratch2(c, 64 * pc->R * sizeof(fe), (void **)&coef));
+    return rs_encode(c, d, pc->R, 64, out, pc->S, coef);
+}
+
+// the mask slice of l or q (out) from the M values in buf, on context x
+static int encode_mask(vg_pc *pc, vg_ctx *x, DevBuf &buf, fe *out)
+{
+    fe *coef;
+    VG_TRY(vg_scratch2(x, pc->M * sizeof(fe), (void **)&coef));
+    return rs_encode(x, pc->F(buf), pc->M, 1, out, pc->S, coef);
+}
+
+static int encode_private(vg_pc *pc, const vg_fe *priv, int log_len, const vg_fe *mask, long n_mask, long *mask_len)
+{
+    VG_TRY(start_private(pc, priv, log_len, mask, n_mask));
+    VG_TRY(encode_data(pc, priv, pc->F(pc->l_eval)));
+    VG_TRY(device_mask(pc, pc->mask, mask, n_mask, pc->M));
+    VG_TRY(encode_mask(pc, pc->ctx, pc->mask, pc->F(pc->l_eval) + 64 * pc->S));
+    if (mask_len) *mask_len = pc->M;
     pc->have_private = true;
     return VG_OK;
 }
@@ -353,7 +382,7 @@ static int encode_private(vg_pc *pc, const vg_fe *priv, int log_len, const vg_fe
 extern "C" int vg_pc_encode_private(vg_pc *pc, const vg_fe *priv, int log_len, const vg_fe *mask, long n_mask,
                                     long *mask_len)
 {
-    return encode_private(pc, priv, log_len, mask, n_mask, mask_len, nullptr);
+    return encode_private(pc, priv, log_len, mask, n_mask, mask_len);
 }
 
 long vg_pc_mask_len(int log_len, long n_pri_mask)
@@ -362,72 +391,73 @@ long vg_pc_mask_len(int log_len, long n_pri_mask)
     return S / mask_gap(S, n_pri_mask);
 }
 
-// <l, q> to res_dev[0] and all_sum to res_dev[1 .. 65]
-static int encode_public(vg_pc *pc, const vg_fe *pub, const vg_fe *pub_mask, long n_mask, fe *res_dev, fe *staging)
+// checks and buffers of the public half
+static int start_public(vg_pc *pc, const vg_fe *pub, const vg_fe *pub_mask, long n_mask)
 {
     if (!pc || !pub || !pub_mask) return vg_fail(VG_ERR_ARG, "vg_pc_encode_public: null argument");
-    if (!pc->have_private) return vg_fail(VG_ERR_STATE, "commit_public before commit_private");
     if (n_mask > pc->M) return vg_fail(VG_ERR_ARG, "public mask longer than the padded private mask (%ld > %ld)", n_mask, pc->M);
     if (pc->gap == 1) return vg_fail(VG_ERR_ARG, "mask fills the whole slice (mask_position_gap == 1)");
     vg_ctx *c = pc->ctx;
-    const long S = pc->S, R = pc->R, M = pc->M, N = 1L << pc->log_len;
-    const int logS = ilog2l(S);
-    const long lq_len = 64 * 2 * R + 2 * M;
-    VG_TRY(ensure(c, pc->q_eval, 65 * S * sizeof(fe)));
-    VG_TRY(ensure(c, pc->h_eval, 65 * S * sizeof(fe)));
-    VG_TRY(ensure(c, pc->vo, 65 * S * sizeof(fe)));
+    const long lq_len = 64 * 2 * pc->R + 2 * pc->M;
+    for (DevBuf *b : {&pc->q_eval, &pc->h_eval, &pc->vo}) VG_TRY(ensure(c, *b, 65 * pc->S * sizeof(fe)));
     VG_TRY(ensure(c, pc->lq, lq_len * sizeof(fe)));
     VG_TRY(ensure(c, pc->lqc, lq_len * sizeof(fe)));
-    fe *l_eval = pc->F(pc->l_eval), *q_eval = pc->F(pc->q_eval), *h_eval = pc->F(pc->h_eval);
-    fe *lq = pc->F(pc->lq), *lqc = pc->F(pc->lqc);
+    return VG_OK;
+}
 
-    const fe *pub_d;
-    VG_TRY(device_input(pc, pub, N, &pub_d));
-    fe *coef;
-    VG_TRY(vg_scratch2(c, 64 * R * sizeof(fe), (void **)&coef));
-    VG_TRY(rs_encode(c, pub_d, R, 64, q_eval, S, coef));
-    DevBuf &mbuf = staging ? pc->mask2 : pc->mask;   // the deferred proof keeps the private mask
-    VG_TRY(device_mask(pc, mbuf, pub_mask, n_mask, M, staging));
-    VG_TRY(rs_encode(c, pc->F(mbuf), M, 1, q_eval + 64 * S, S, coef));
+// Slices slice0 .. slice0 + count - 1 of h and the virtual oracle, with their
+// all_sum entries, from those of l and q, on context x: the samples of l q at
+// 2 m points (m = R for data slices, M for the mask), their interpolation, the
+// quotient's encoding and the oracle.
+static int quotient(vg_pc *pc, vg_ctx *x, int slice0, int count, long m, fe *sums)
+{
+    const long S = pc->S;
+    const int logS = ilog2l(S), l2m = ilog2l(2 * m);
+    fe *l = pc->F(pc->l_eval) + slice0 * S, *q = pc->F(pc->q_eval) + slice0 * S, *h = pc->F(pc->h_eval) + slice0 * S;
+    fe *lq = pc->F(pc->lq) + slice0 * 2 * pc->R, *lqc = pc->F(pc->lqc) + slice0 * 2 * pc->R;
+    k_lq_sample<<<std::min<unsigned>(grid_for(2 * m * count, 256), 148u * 8u), 256, 0, x->stream>>>(l, q, S, m, S / (2 * m),
+                                                                                                   count, lq);
+    VG_LAUNCHED(x);
+    VG_TRY(vg_ntt(x, (const vg_fe *)lq, 2 * m, 2 * m, (vg_fe *)lqc, l2m, 2 * m, count, to_vg(vg::fe_inv(root_of(l2m))), 1));
+    VG_TRY(vg_ntt(x, (const vg_fe *)(lqc + m), m, 2 * m, (vg_fe *)h, logS, S, count, to_vg(root_of(logS)), 0));
+    const fe *tf_lo, *tf_hi, *ti_lo, *ti_hi;
+    VG_TRY(vg_twiddles(x, root_of(logS), logS, &tf_lo, &tf_hi));
+    VG_TRY(vg_twiddles(x, vg::fe_inv(root_of(logS)), logS, &ti_lo, &ti_hi));
+    {
+        ProfScope ps(x, KF_VIRTUAL_ORACLE, 64.0 * (double)count * (double)S);
+        k_virtual_oracle<<<std::min<unsigned>(grid_for(count * S, 256), 148u * 16u), 256, 0, x->stream>>>(
+            pc->F(pc->l_eval), pc->F(pc->q_eval), pc->F(pc->h_eval), lqc, S, m, logS, slice0, count, tf_lo, tf_hi, ti_lo,
+            ti_hi, pc->F(pc->vo));
+    }
+    VG_LAUNCHED(x);
+    k_all_sum<<<1, 64, 0, x->stream>>>(lqc, m, slice0, count, sums);
+    VG_LAUNCHED(x);
+    return VG_OK;
+}
 
-    // inner product check value
+// the sampled <l, q> (every slice encoded) to res_dev[0]
+static int inner_product(vg_pc *pc, fe *res_dev)
+{
+    vg_ctx *c = pc->ctx;
     fe *parts;
     const int nb = 148 * 4;
     VG_TRY(vg_partials(c, nb, &parts));
-    k_inner_product<<<nb, 256, 0, c->stream>>>(l_eval, q_eval, S, pc->gap, parts);
+    k_inner_product<<<nb, 256, 0, c->stream>>>(pc->F(pc->l_eval), pc->F(pc->q_eval), pc->S, pc->gap, parts);
     VG_LAUNCHED(c);
-    VG_TRY(vg_reduce_partials(c, parts, nb, 1, res_dev));
+    return vg_reduce_partials(c, parts, nb, 1, res_dev);
+}
 
-    // lq samples, their interpolation and the quotient h
-    fe *lq_m = lq + 64 * 2 * R, *lqc_m = lqc + 64 * 2 * R;
-    k_lq_sample<<<148 * 8, 256, 0, c->stream>>>(l_eval, q_eval, S, R, S / (2 * R), 64, lq);
-    VG_LAUNCHED(c);
-    k_lq_sample<<<grid_for(2 * M, 256), 256, 0, c->stream>>>(l_eval + 64 * S, q_eval + 64 * S, S, M, S / (2 * M), 1, lq_m);
-    VG_LAUNCHED(c);
-    int l2R = ilog2l(2 * R), l2M = ilog2l(2 * M);
-    VG_TRY(vg_ntt(c, (const vg_fe *)lq, 2 * R, 2 * R, (vg_fe *)lqc, l2R, 2 * R, 64, to_vg(vg::fe_inv(root_of(l2R))), 1));
-    VG_TRY(vg_ntt(c, (const vg_fe *)lq_m, 2 * M, 2 * M, (vg_fe *)lqc_m, l2M, 2 * M, 1, to_vg(vg::fe_inv(root_of(l2M))), 1));
-    VG_TRY(vg_ntt(c, (const vg_fe *)(lqc + R), R, 2 * R, (vg_fe *)h_eval, logS, S, 64, to_vg(root_of(logS)), 0));
-    VG_TRY(vg_ntt(c, (const vg_fe *)(lqc_m + M), M, 2 * M, (vg_fe *)(h_eval + 64 * S), logS, S, 1, to_vg(root_of(logS)), 0));
-
-    // virtual oracle and all_sum
-    const fe *tf_lo, *tf_hi, *ti_lo, *ti_hi;
-    VG_TRY(vg_twiddles(c, root_of(logS), logS, &tf_lo, &tf_hi));
-    VG_TRY(vg_twiddles(c, vg::fe_inv(root_of(logS)), logS, &ti_lo, &ti_hi));
-    {
-        ProfScope ps(c, KF_VIRTUAL_ORACLE, 64.0 * 64.0 * (double)S);
-        k_virtual_oracle<<<148 * 16, 256, 0, c->stream>>>(l_eval, q_eval, h_eval, lqc, S, R, logS, 0, 64,
-                                                          tf_lo, tf_hi, ti_lo, ti_hi, pc->F(pc->vo));
-    }
-    VG_LAUNCHED(c);
-    k_virtual_oracle<<<grid_for(S, 256), 256, 0, c->stream>>>(l_eval, q_eval, h_eval, lqc_m, S, M, logS, 64, 1,
-                                                             tf_lo, tf_hi, ti_lo, ti_hi, pc->F(pc->vo));
-    VG_LAUNCHED(c);
-    fe *sums_d = res_dev + 1;
-    k_all_sum<<<1, 64, 0, c->stream>>>(lqc, R, 0, 64, sums_d);
-    VG_LAUNCHED(c);
-    k_all_sum<<<1, 1, 0, c->stream>>>(lqc_m, M, 64, 1, sums_d);
-    VG_LAUNCHED(c);
+// <l, q> to res_dev[0] and all_sum to res_dev[1 .. 65]
+static int encode_public(vg_pc *pc, const vg_fe *pub, const vg_fe *pub_mask, long n_mask, fe *res_dev)
+{
+    if (!pc->have_private) return vg_fail(VG_ERR_STATE, "commit_public before commit_private");
+    VG_TRY(start_public(pc, pub, pub_mask, n_mask));
+    VG_TRY(encode_data(pc, pub, pc->F(pc->q_eval)));
+    VG_TRY(device_mask(pc, pc->mask, pub_mask, n_mask, pc->M));
+    VG_TRY(encode_mask(pc, pc->ctx, pc->mask, pc->F(pc->q_eval) + 64 * pc->S));
+    VG_TRY(inner_product(pc, res_dev));
+    VG_TRY(quotient(pc, pc->ctx, 0, 64, pc->R, res_dev + 1));
+    VG_TRY(quotient(pc, pc->ctx, 64, 1, pc->M, res_dev + 1));
     pc->have_public = true;
     return VG_OK;
 }
@@ -435,10 +465,10 @@ static int encode_public(vg_pc *pc, const vg_fe *pub, const vg_fe *pub_mask, lon
 extern "C" int vg_pc_encode_public(vg_pc *pc, const vg_fe *pub, const vg_fe *pub_mask, long n_mask, vg_fe *all_sum,
                                    vg_fe *inner_product)
 {
-    if (!pc || !all_sum) return vg_fail(VG_ERR_ARG, "vg_pc_encode_public: null argument");
+    if (!pc || !all_sum || !pub || !pub_mask) return vg_fail(VG_ERR_ARG, "vg_pc_encode_public: null argument");
     vg_ctx *c = pc->ctx;
     VG_TRY(ensure(c, pc->res, 66 * sizeof(fe)));
-    VG_TRY(encode_public(pc, pub, pub_mask, n_mask, pc->F(pc->res), nullptr));
+    VG_TRY(encode_public(pc, pub, pub_mask, n_mask, pc->F(pc->res)));
     fe *host;
     VG_TRY(vg_pinned(c, 66, &host));
     VG_CHECK_CUDA(cudaMemcpyAsync(host, pc->res.p, 66 * sizeof(fe), cudaMemcpyDeviceToHost, c->stream));
@@ -621,6 +651,105 @@ static int ensure_pinned(vg_pc *pc, size_t elems)
     return VG_OK;
 }
 
+// The second stream of a whole commitment.  Everything about the mask slices
+// (single transforms, all latency, some 100 us in a row) runs there beside the
+// data slices.  From BESIDE_MIN on the hash chains of l, a third of the hashing,
+// run there too while the first stream takes in and encodes the public half
+// (2^20 values from host memory 20.1 -> 18.7 ms); for small commitments they
+// only slow the short kernels of the first stream down (2^15 903 -> 1120 us).
+// Every buffer belongs to the first stream: the second one starts after what
+// is queued there (fork) and the first continues after it (join) before
+// anything is reused or freed; an error in between waits for the second stream
+// instead.  While the context's launches are profiled everything stays on its
+// own stream.
+constexpr long BESIDE_MIN = 1L << 19;
+struct SideJoin {
+    vg_ctx *c, *x;
+    bool count;   // the second stream's launches are counted with the first's (a lent context counts its own)
+    long long launches0 = 0;
+    std::vector<cudaEvent_t> events;
+    bool forked = false;
+    SideJoin(vg_ctx *ctx, vg_ctx *side, bool own) : c(ctx), x(side ? side : ctx), count(side && own), launches0(x->launches) {}
+    ~SideJoin()
+    {
+        if (forked) cudaStreamSynchronize(x->stream);
+        if (count) c->launches += x->launches - launches0;
+        for (cudaEvent_t e : events) cudaEventDestroy(e);
+    }
+    int mark(vg_ctx *on, cudaEvent_t *e)
+    {
+        *e = nullptr;
+        if (x == c) return VG_OK;
+        VG_CHECK_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        events.push_back(*e);
+        VG_CHECK_CUDA(cudaEventRecord(*e, on->stream));
+        return VG_OK;
+    }
+    int wait(vg_ctx *on, cudaEvent_t e)
+    {
+        if (e) VG_CHECK_CUDA(cudaStreamWaitEvent(on->stream, e, 0));
+        return VG_OK;
+    }
+    int wait_for(vg_ctx *waiter, vg_ctx *signaler)
+    {
+        cudaEvent_t e;
+        VG_TRY(mark(signaler, &e));
+        return wait(waiter, e);
+    }
+    int fork()
+    {
+        VG_TRY(wait_for(x, c));
+        forked = x != c;
+        return VG_OK;
+    }
+    int join()
+    {
+        VG_TRY(wait_for(c, x));
+        forked = false;
+        return VG_OK;
+    }
+};
+
+// pc->side ready for use
+static int commit_streams(vg_pc *pc)
+{
+    vg_ctx *c = pc->ctx;
+    if (!pc->side) {
+        VG_TRY(vg_ctx_create(c->device, &pc->side));
+        pc->own_side = true;
+    }
+    pc->side->hash_kind = c->hash_kind;
+    return VG_OK;
+}
+
+void vg_pc_set_side(vg_pc *pc, vg_ctx *side)
+{
+    if (!pc || pc->own_side) return;
+    pc->side = side;
+}
+
+struct LeafSet {
+    const fe *cw;
+    long n;
+    uint64_t *tree;
+};
+static int leaf_sets(vg_ctx *x, const std::vector<LeafSet> &sets)
+{
+    for (size_t b = 0; b < sets.size(); b += MAX_HASH_JOBS) {
+        ChainJobs cj{};
+        cj.slices = 65;
+        long total = 0;
+        for (size_t k = b; k < sets.size() && k < b + MAX_HASH_JOBS; ++k) {
+            const long nleaves = sets[k].n >> 1;
+            cj.j[cj.count++] = {sets[k].cw, sets[k].n, sets[k].tree + 4 * nleaves, total};
+            total += nleaves;
+        }
+        cj.total = total;
+        VG_TRY(vg_leaf_chains(x, cj));
+    }
+    return VG_OK;
+}
+
 int vg_pc_prove_deferred(vg_pc *pc, const vg_fe *priv, int log_len, const vg_fe *pri_mask, long n_pri_mask,
                          const vg_fe *pub, const vg_fe *pub_mask, long n_pub_mask, const vg_fe *fri_r, int nlevels,
                          int nq, const int *which, const long *pos, vg_pc_results *out)
@@ -646,25 +775,58 @@ int vg_pc_prove_deferred(vg_pc *pc, const vg_fe *priv, int log_len, const vg_fe 
     fe *h_mask = pc->hpin, *h_in = h_mask + e_masks, *h_res = h_in + e_in, *h_roots = h_res + e_res,
        *h_final = h_roots + e_roots, *h_qv = h_final + e_final, *h_qp = h_qv + e_qv;
 
-    // commitment of the private and public inputs, virtual oracle
-    long Mp = 0;
-    VG_TRY(encode_private(pc, priv, log_len, pri_mask, n_pri_mask, &Mp, h_mask));
-    if (Mp != M) return vg_fail(VG_ERR_STATE, "mask length %ld != %ld", Mp, M);
-    if (n_pub_mask > M) return vg_fail(VG_ERR_ARG, "public mask longer than the padded private mask (%ld > %ld)", n_pub_mask, M);
+    // sizes, checks and every buffer first: the second stream uses them too
+    VG_TRY(start_private(pc, priv, log_len, pri_mask, n_pri_mask));
+    if (pc->M != M) return vg_fail(VG_ERR_STATE, "mask length %ld != %ld", pc->M, M);
+    VG_TRY(start_public(pc, pub, pub_mask, n_pub_mask));
+    VG_TRY(ensure(c, pc->mask, M * sizeof(fe)));
+    VG_TRY(ensure(c, pc->mask2, M * sizeof(fe)));
     VG_TRY(ensure(c, pc->res, 66 * sizeof(fe)));
-    VG_TRY(encode_public(pc, pub, pub_mask, n_pub_mask, pc->F(pc->res), h_mask + M));
+    VG_TRY(ensure(c, pc->tree_l, (size_t)S * 32));
+    VG_TRY(ensure(c, pc->tree_h, (size_t)S * 32));
+    VG_TRY(ensure(c, pc->roots, ndesc * 32));
+    if ((int)pc->levels.size() < nlevels) pc->levels.resize(nlevels);
+    for (int t = 0; t < nlevels; ++t) {
+        PcLevel &L = pc->levels[t];
+        L.n = S >> (t + 1);
+        VG_TRY(ensure(c, L.cw, 65 * L.n * sizeof(fe)));
+        VG_TRY(ensure(c, L.tree, L.n * 32));
+    }
+    if (!c->profiling) VG_TRY(commit_streams(pc));
+    SideJoin side(c, c->profiling ? nullptr : pc->side, pc->own_side);
+    vg_ctx *x = side.x;
+    VG_TRY(side.fork());
+    // second stream: the mask slices, end to end (single transforms, all latency)
+    fe *l_eval = pc->F(pc->l_eval), *res = pc->F(pc->res);
+    VG_TRY(stage_mask(x, pc->mask, pri_mask, n_pri_mask, M, h_mask));
+    VG_TRY(encode_mask(pc, x, pc->mask, l_eval + 64 * S));
+    VG_TRY(stage_mask(x, pc->mask2, pub_mask, n_pub_mask, M, h_mask + M));
+    VG_TRY(encode_mask(pc, x, pc->mask2, pc->F(pc->q_eval) + 64 * S));
+    VG_TRY(quotient(pc, x, 64, 1, M, res + 1));
+    cudaEvent_t masks = nullptr;
+    VG_TRY(side.mark(x, &masks));
+    // the private data; then its leaf chains on the second stream, beside the rest
+    VG_TRY(encode_data(pc, priv, l_eval));
+    pc->have_private = true;
+    const bool l_beside = x != c && S >= BESIDE_MIN;
+    if (l_beside) {
+        VG_TRY(side.wait_for(x, c));
+        VG_TRY(leaf_sets(x, {{l_eval, S, pc->U(pc->tree_l)}}));
+    }
+    // the public data, the quotient and the virtual oracle
+    VG_TRY(encode_data(pc, pub, pc->F(pc->q_eval)));
+    VG_TRY(quotient(pc, c, 0, 64, pc->R, res + 1));
+    VG_TRY(side.wait(c, masks));
+    VG_TRY(inner_product(pc, res));
+    pc->have_public = true;
 
     // FRI folds, level by level (fri.cpp:321-340, 367-379)
     const int logS = ilog2l(S);
     const fe *ti_lo, *ti_hi;
     VG_TRY(vg_twiddles(c, vg::fe_inv(root_of(logS)), logS, &ti_lo, &ti_hi));
-    if ((int)pc->levels.size() < nlevels) pc->levels.resize(nlevels);
     for (int t = 0; t < nlevels; ++t) {
         const long n = S >> t;
         PcLevel &L = pc->levels[t];
-        L.n = n >> 1;
-        VG_TRY(ensure(c, L.cw, 65 * L.n * sizeof(fe)));
-        VG_TRY(ensure(c, L.tree, L.n * 32));
         const fe *in = t == 0 ? pc->F(pc->vo) : pc->F(pc->levels[t - 1].cw);
         const long total = 65 * L.n;
         {
@@ -676,30 +838,17 @@ int vg_pc_prove_deferred(vg_pc *pc, const vg_fe *priv, int log_len, const vg_fe 
     }
     pc->nlevels = nlevels;
 
-    // every leaf chain, then every Merkle tree, batched (fri.cpp:394-420, merkle_tree.cpp)
-    VG_TRY(ensure(c, pc->tree_l, (size_t)S * 32));
-    VG_TRY(ensure(c, pc->tree_h, (size_t)S * 32));
-    VG_TRY(ensure(c, pc->roots, ndesc * 32));
-    struct Set { const fe *cw; long n; uint64_t *tree; };
-    std::vector<Set> sets;
-    sets.push_back({pc->F(pc->l_eval), S, pc->U(pc->tree_l)});
+    // the other leaf chains in one launch, then every Merkle tree, batched (fri.cpp:394-420, merkle_tree.cpp)
+    std::vector<LeafSet> sets;
+    sets.push_back({l_eval, S, pc->U(pc->tree_l)});
     sets.push_back({pc->F(pc->h_eval), S, pc->U(pc->tree_h)});
     for (int t = 0; t < nlevels; ++t) sets.push_back({pc->F(pc->levels[t].cw), pc->levels[t].n, pc->U(pc->levels[t].tree)});
-    for (size_t b = 0; b < sets.size(); b += MAX_HASH_JOBS) {
-        ChainJobs cj{};
-        cj.slices = 65;
-        long total = 0;
-        for (size_t k = b; k < sets.size() && k < b + MAX_HASH_JOBS; ++k) {
-            const long nleaves = sets[k].n >> 1;
-            cj.j[cj.count++] = {sets[k].cw, sets[k].n, sets[k].tree + 4 * nleaves, total};
-            total += nleaves;
-        }
-        cj.total = total;
-        VG_TRY(vg_leaf_chains(c, cj));
-    }
+    VG_TRY(leaf_sets(c, std::vector<LeafSet>(sets.begin() + (l_beside ? 1 : 0), sets.end())));
+    VG_TRY(side.join());
     for (size_t b = 0; b < sets.size(); b += MAX_HASH_JOBS) {
         TreeJobs tj{};
-        for (size_t k = b; k < sets.size() && k < b + MAX_HASH_JOBS; ++k) tj.t[tj.count++] = {sets[k].tree, sets[k].n >> 1, sets[k].n >> 1};
+        for (size_t k = b; k < sets.size() && k < b + MAX_HASH_JOBS; ++k)
+            tj.t[tj.count++] = {sets[k].tree, sets[k].n >> 1, sets[k].n >> 1};
         VG_TRY(vg_merkle_trees(c, tj, pc->U(pc->roots) + 4 * b));
     }
 

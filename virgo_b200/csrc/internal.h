@@ -77,6 +77,10 @@ struct vg_pc_results {
 };
 // Mask length M the private mask is padded to (poly_commit.h:66-70).
 long vg_pc_mask_len(int log_len, long n_pri_mask);
+// Lends pc the context of its second stream (same device; it must outlive pc
+// or be replaced by null), used only inside vg_pc_prove_deferred and joined
+// before it returns.
+void vg_pc_set_side(vg_pc *pc, vg_ctx *side);
 // The whole commitment of one proof: RS encodings of the private input and of
 // the public eq table, the virtual oracle, every FRI fold (challenges fri_r),
 // all leaf chains and Merkle trees batched, the query answers for

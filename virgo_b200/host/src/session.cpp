@@ -149,6 +149,15 @@ struct vg_session {
     PassResults last;
 };
 
+// the session's third stream: the commitment's second one, then the side proof's
+static int third_stream(vg_session *s)
+{
+    if (s->fctx) return VG_OK;
+    int dev = 0;
+    vg_ctx_device(s->ctx, &dev);
+    return vg_ctx_create(dev, &s->fctx);
+}
+
 // The verifier runs `./fft_gkr <L - 6>` next to every proof of input size
 // 2^L and counts its prover time (vpd_verifier.cpp:89-99); its random stream
 // is that of a fresh process (seed 1).  Here it is launched on the session's
@@ -159,13 +168,8 @@ static int fft_side_launch(vg_session *s, int *lg_out)
     *lg_out = 0;
     const int lg = s->circuit->C.circuit[0].bit_length - 6;
     if (!s->fft_on || lg < 1) return VG_OK;
-    int rc = VG_OK;
-    if (!s->fctx) {
-        int dev = 0;
-        vg_ctx_device(s->ctx, &dev);
-        rc = vg_ctx_create(dev, &s->fctx);
-        if (rc != VG_OK) return rc;
-    }
+    int rc = third_stream(s);
+    if (rc != VG_OK) return rc;
     if (!s->fft) {
         rc = vg_fft_gkr_create(s->fctx, lg, &s->fft);
         if (rc != VG_OK) return rc;
@@ -783,7 +787,10 @@ static int prove_pass(vg_session *s, unsigned seed, bool launch, PassResults &re
         }
         // the commitment depends on no GKR device result: it runs on its own
         // stream, concurrently with the sumcheck work enqueued above
-        int rc = vg_eq_table_async(s->cctx, (const vg_fe *)r_0.data(), L, (vg_fe *)s->pub);
+        int rc = third_stream(s);
+        if (rc != VG_OK) return rc;
+        vg_pc_set_side(s->pc, s->fctx);
+        rc = vg_eq_table_async(s->cctx, (const vg_fe *)r_0.data(), L, (vg_fe *)s->pub);
         if (rc == VG_OK)
             rc = vg_pc_prove_deferred(s->pc, (const vg_fe *)p.circuit_value[0], L, (const vg_fe *)p.all_pri_mask.data(),
                                       (long)p.all_pri_mask.size(), (const vg_fe *)s->pub,
