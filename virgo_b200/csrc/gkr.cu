@@ -561,6 +561,21 @@ struct EdgeView {
     const uint32_t *off, *g, *o;
     const uint16_t *tk;
 };
+struct EdgeRec {
+    uint32_t g, o;
+    int tk;
+};
+// edge p's record if p < end
+__device__ __forceinline__ EdgeRec load_rec(const EdgeView &e, uint32_t p, uint32_t end)
+{
+    EdgeRec r{0, 0, 0};
+    if (p < end) {
+        r.g = e.g[p];
+        r.o = e.o[p];
+        r.tk = e.tk[p];
+    }
+    return r;
+}
 
 // One thread per key with at most LIGHT_MAX edges; out_m / out_v are the
 // add_mult_sum and addV_array tables.
@@ -602,7 +617,13 @@ __global__ void __launch_bounds__(GKR_THREADS) k_gather_long(EdgeView e, const u
         const uint32_t k = keys[w], s = e.off[k], t = e.off[k + 1];
         if (PH == 0) {
             fe am = vg::fe_zero(), av = vg::fe_zero();
-            for (uint32_t p = s + lane; p < t; p += 32) edge1(e.tk[p], e.g[p], e.o[p], bg, prev, am, av);
+            EdgeRec r = load_rec(e, s + lane, t), r2 = load_rec(e, s + lane + 32, t);   // two steps ahead
+            for (uint32_t p = s + lane; p < t; p += 32) {
+                const EdgeRec x = r;
+                r = r2;
+                r2 = load_rec(e, p + 64, t);
+                edge1(x.tk, x.g, x.o, bg, prev, am, av);
+            }
             am = warp_sum(am);
             av = warp_sum(av);
             if (lane == 0) {
@@ -612,7 +633,13 @@ __global__ void __launch_bounds__(GKR_THREADS) k_gather_long(EdgeView e, const u
         } else {
             fe a[4] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
             unsigned used = 0;
-            for (uint32_t p = s + lane; p < t; p += 32) edge2(e.tk[p], e.g[p], e.o[p], bg, bu, a, used);
+            EdgeRec r = load_rec(e, s + lane, t), r2 = load_rec(e, s + lane + 32, t);   // two steps ahead
+            for (uint32_t p = s + lane; p < t; p += 32) {
+                const EdgeRec x = r;
+                r = r2;
+                r2 = load_rec(e, p + 64, t);
+                edge2(x.tk, x.g, x.o, bg, bu, a, used);
+            }
 #pragma unroll
             for (int q = 0; q < 4; ++q) a[q] = warp_sum(a[q]);
             used = __reduce_or_sync(0xffffffffu, used);
@@ -1238,29 +1265,58 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_gather_round2(Gather
     const bool hi = lane & 1;
     const long nwarps = (long)gridDim.x * (THREADS / 32), w0 = (blockIdx.x * (long)THREADS + threadIdx.x) >> 5;
     fe sa[3] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero()}, sb[3] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
-    for (long w = w0; w < (nquads >> 5); w += nwarps) {
+    // Key offsets run two halves (64 keys) ahead and the first edge's record one
+    // half ahead, so a half waits for its operands only, not for offset, record
+    // and operands one after the other.
+    const long nblk = nquads >> 5;
+    auto keys_of = [&](long w, int h) { return 128 * w + 64 * h + 2 * lane; };
+    auto offsets = [&](long k0, uint32_t (&o)[3]) {
+        const uint2 x = *reinterpret_cast<const uint2 *>(ga.e.off + k0);
+        o[0] = x.x;
+        o[1] = x.y;
+        o[2] = ga.e.off[k0 + 2];
+    };
+    uint32_t cur[3] = {0, 0, 0}, nxt[3] = {0, 0, 0};
+    EdgeRec rec{};
+    if (w0 < nblk) {
+        offsets(keys_of(w0, 0), cur);
+        offsets(keys_of(w0, 1), nxt);
+        rec = load_rec(ga.e, cur[0], cur[2]);
+    }
+    for (long w = w0; w < nblk; w += nwarps) {
         fe v[2], a[2], m[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const long k0 = 128 * w + 64 * h + 2 * lane;
+            const long k0 = keys_of(w, h);
+            const EdgeRec first = rec;
+            const uint32_t s0 = cur[0], s1 = cur[1], s2 = cur[2];
+            rec = load_rec(ga.e, nxt[0], nxt[2]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) cur[k] = nxt[k];
+            if (w + nwarps < nblk) offsets(keys_of(w + nwarps, h), nxt);
+            else nxt[0] = nxt[2] = 0;   // no edges
             fe av[2], am[2];
-            uint32_t s = ga.e.off[k0];
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                const uint32_t t = ga.e.off[k0 + k + 1];
+                const uint32_t s = k ? s1 : s0, t = k ? s2 : s1;
                 if (t - s > (uint32_t)LIGHT_MAX) {
                     am[k] = ga.tm[k0 + k];
                     av[k] = ga.tv[k0 + k];
                 } else if (PH == 0) {
                     am[k] = av[k] = vg::fe_zero();
-                    for (uint32_t p = s; p < t; ++p) edge1(ga.e.tk[p], ga.e.g[p], ga.e.o[p], ga.bg, ga.prev, am[k], av[k]);
+                    for (uint32_t p = s; p < t; ++p) {
+                        const EdgeRec e = p == s0 ? first : load_rec(ga.e, p, p + 1);
+                        edge1(e.tk, e.g, e.o, ga.bg, ga.prev, am[k], av[k]);
+                    }
                 } else {
                     fe q[4] = {vg::fe_zero(), vg::fe_zero(), vg::fe_zero(), vg::fe_zero()};
                     unsigned used = 0;
-                    for (uint32_t p = s; p < t; ++p) edge2(ga.e.tk[p], ga.e.g[p], ga.e.o[p], ga.bg, ga.bu, q, used);
+                    for (uint32_t p = s; p < t; ++p) {
+                        const EdgeRec e = p == s0 ? first : load_rec(ga.e, p, p + 1);
+                        edge2(e.tk, e.g, e.o, ga.bg, ga.bu, q, used);
+                    }
                     phase2_out(q, used, vu, am[k], av[k]);
                 }
-                s = t;
             }
             fe v0, v1;
             ld_pair(xV + k0, v0, v1);   // layer values: real parts
