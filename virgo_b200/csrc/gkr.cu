@@ -127,37 +127,37 @@ __global__ void k_eval_layer(const uint8_t *__restrict__ ty, const uint32_t *__r
 }
 
 // ------------------------------------------------------------ eq tables
-// out[i] = scale * prod_{b < nbits} (bit b of i ? r[b] : 1 - r[b])
-__global__ void k_eq_half(const fe *__restrict__ r, int nbits, fe scale, fe *__restrict__ out)
-{
-    long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (i >= (1L << nbits)) return;
-    fe x = scale;
-    for (int b = 0; b < nbits; ++b) x = x * (((i >> b) & 1) ? r[b] : vg::fe_one() - r[b]);
-    out[i] = x;
-}
-
 // Several half tables in one launch (the tables of a phase init are built
-// together): table q covers threads [begin[q], begin[q + 1]).
+// together): table q covers threads [begin[q], begin[q + 1]), its entry i goes
+// to out[q][step[q] i].  The point's coordinates travel as kernel arguments
+// (copies to the device between the phases' kernels cost more than the
+// tables).  One more thread forms phase 2's v_u = V(r_u) + mask term, the
+// folded V pair of the last phase-1 round at r (zk_prover.cpp:796-797),
+// where the pair is, so phase 2 can start without the host reading it first.
 struct EqJobs {
-    const fe *r[4];
+    fe r[4][16];
     fe *out[4];
     fe scale[4];
-    int nbits[4];
+    int nbits[4], step[4];
     long begin[5];
     int count;
+    const fe *last6;   // null: no v_u
+    fe vu_r, vu_add;
+    fe *vu;
 };
-__global__ void k_eq_halves(EqJobs J)
+__global__ void k_eq_halves(const __grid_constant__ EqJobs J)
 {
     const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (t >= J.begin[J.count]) return;
+    if (t >= J.begin[J.count]) {
+        if (t == J.begin[J.count] && J.last6) *J.vu = vg::fe_fma(J.last6[0], J.vu_r, J.last6[1] - J.last6[0]) + J.vu_add;
+        return;
+    }
     int q = 0;
     while (t >= J.begin[q + 1]) ++q;
     const long i = t - J.begin[q];
-    const fe *r = J.r[q];
-    fe x = J.scale[q];
-    for (int b = 0; b < J.nbits[q]; ++b) x = x * (((i >> b) & 1) ? r[b] : vg::fe_one() - r[b]);
-    J.out[q][i] = x;
+    fe x[2] = {J.scale[q], vg::fe_one()};   // two chains of products side by side
+    for (int b = 0; b < J.nbits[q]; ++b) x[b & 1] = x[b & 1] * (((i >> b) & 1) ? J.r[q][b] : vg::fe_one() - J.r[q][b]);
+    J.out[q][J.step[q] * i] = x[0] * x[1];
 }
 
 // out[x] = lo[x & mask] * hi[x >> fh]
@@ -244,8 +244,18 @@ __global__ void __launch_bounds__(MLE_THREADS) k_mle(const fe *__restrict__ vals
 }
 
 // ---------------------------------------------------------- accumulators
+// Entries 2k, 2k + 1 of a table in one 32-byte load (p 32-byte aligned)
+__device__ __forceinline__ void ld_pair(const fe *p, fe &x0, fe &x1)
+{
+    asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];"
+        : "=l"(x0.img), "=l"(x0.real), "=l"(x1.img), "=l"(x1.real)
+        : "l"(p));
+}
+// beta_g(i) = alpha eq(r0, i) + beta eq(r1, i) from half tables, the two
+// points' entries side by side: a random i then touches two lines, not four
+// (the gathers over scattered gates are bound by the lines L1 looks up)
 struct BetaG {
-    const fe *f0, *s0, *f1, *s1;   // alpha*eq(r0 low half), eq(r0 high half), beta*..., eq(r1 high)
+    const fe *f, *s;   // {alpha eq(r0), beta eq(r1)} over the low bits, {eq(r0), eq(r1)} over the high ones
     int fh;
     long mask;
     // the layer's values by gate: phase 1's gathers store each gate's value
@@ -255,7 +265,10 @@ struct BetaG {
     __device__ __forceinline__ fe at(long i) const
     {
         if (tab) return tab[i];
-        return vg::fe_dot2(f0[i & mask], s0[i >> fh], f1[i & mask], s1[i >> fh]);
+        fe f0, f1, s0, s1;
+        ld_pair(f + 2 * (i & mask), f0, f1);
+        ld_pair(s + 2 * (i >> fh), s0, s1);
+        return vg::fe_dot2(f0, s0, f1, s1);
     }
 };
 struct BetaU {
@@ -1014,14 +1027,6 @@ __global__ void k_predicates_relay(fe *__restrict__ out, const fe *__restrict__ 
     out[10] = out[10] * (bv_lo[0] * bv_hi[0]);
 }
 
-// v_u = V(r_u) + mask term: the folded V pair of the last phase-1 round at r
-// (zk_prover.cpp:796-797), computed where the pair is, so phase 2 can start
-// without the host reading it first
-__global__ void k_vu(const fe *__restrict__ last6, fe r, fe addend, fe *__restrict__ vu)
-{
-    *vu = (last6[0] + r * (last6[1] - last6[0])) + addend;
-}
-
 // ------------------------------------------------------------ round kernel
 // The sums are reduced over the grid by grid_sum, so one launch returns them.
 // The fold challenge comes from device memory (rp), so a captured launch
@@ -1106,13 +1111,6 @@ __device__ __forceinline__ void round2_finish(const fe (&sa)[3], const fe (&sb)[
     }
 }
 
-// Entries 2k, 2k + 1 of a table in one 32-byte load (p 32-byte aligned)
-__device__ __forceinline__ void ld_pair(const fe *p, fe &x0, fe &x1)
-{
-    asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];"
-        : "=l"(x0.img), "=l"(x0.real), "=l"(x1.img), "=l"(x1.real)
-        : "l"(p));
-}
 __device__ __forceinline__ fe sel_fe(bool c, fe a, fe b) { return c ? a : b; }
 __device__ __forceinline__ fe shfl_xor_fe(fe x, int mask)
 {
@@ -1463,7 +1461,6 @@ struct vg_gkr {
     fe *buf[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};   // ping-pong V, AV, AM
     unsigned long long *acc = nullptr;   // 2 tables x 4 words x 2^max_bl
     fe *eq = nullptr;                    // half tables
-    fe *rbuf = nullptr;                  // challenges (device copy)
     unsigned long long *round_acc = nullptr;   // the round kernels' limb sums over the grid (grid_sum), zero between launches
     fe *round_out = nullptr;             // round sums (3) written by the last block
     unsigned *round_counter = nullptr;   // blocks finished, reset by the last one
@@ -2036,7 +2033,6 @@ extern "C" int vg_gkr_create(vg_ctx *ctx, const vg_circuit *c, vg_gkr **out)
         vg_gkr_destroy(g);
         return vg_fail(VG_ERR_OOM, "vg_gkr_create: %s allocation failed", what);
     };
-    if (cudaMalloc(&g->rbuf, 3 * 64 * sizeof(fe)) != cudaSuccess) return fail("challenges");
     if (cudaMalloc(&g->round_acc, LIMBS * 6 * 8) != cudaSuccess) return fail("round sums");
     if (cudaMalloc(&g->rg_acc, RG_MAX * RG_LIMBS * 8) != cudaSuccess) return fail("group sums");
     if (cudaMalloc(&g->round_out, 16 * sizeof(fe)) != cudaSuccess) return fail("round sums");
@@ -2077,7 +2073,6 @@ extern "C" int vg_gkr_destroy(vg_gkr *g)
         for (int k = 0; k < 3; ++k) cudaFree(g->buf[b][k]);
     cudaFree(g->acc);
     cudaFree(g->eq);
-    cudaFree(g->rbuf);
     cudaFree(g->round_acc);
     cudaFree(g->round_out);
     cudaFree(g->round_counter);
@@ -2145,19 +2140,19 @@ extern "C" int vg_gkr_layer_values(vg_gkr *g, int layer, const vg_fe **dev_value
     return VG_OK;
 }
 
-// eq half tables for bits r[0..len): low half (len >> 1 bits, scaled) and high half
 // Adds the low half (len >> 1 bits, scaled) and the high half of the eq table
-// of r to J; *fh = the low half's bit count.
-static void add_halves(EqJobs &J, const fe *r_dev, int len, fe scale, fe *lo, fe *hi, int *fh)
+// of r (host, at most 30 entries) to J, entries `step` apart; *fh = the low
+// half's bit count.
+static void add_halves(EqJobs &J, const vg_fe *r, int len, fe scale, fe *lo, fe *hi, int *fh, int step = 1)
 {
     const int f = len >> 1, s = len - f;
     const int bits[2] = {f, s};
-    const fe *rs[2] = {r_dev, r_dev + f};
     fe *outs[2] = {lo, hi};
     for (int k = 0; k < 2; ++k) {
         const int q = J.count++;
-        J.r[q] = rs[k];
+        for (int b = 0; b < bits[k]; ++b) J.r[q][b] = tofe(r[(k ? f : 0) + b]);
         J.out[q] = outs[k];
+        J.step[q] = step;
         J.scale[q] = k == 0 ? scale : vg::fe_one();
         J.nbits[q] = bits[k];
         J.begin[q + 1] = J.begin[q] + (1L << bits[k]);
@@ -2165,25 +2160,10 @@ static void add_halves(EqJobs &J, const fe *r_dev, int len, fe scale, fe *lo, fe
     *fh = f;
 }
 
-static int launch_halves(vg_gkr *g, const EqJobs &J)
+static int launch_halves(vg_ctx *c, const EqJobs &J)
 {
-    k_eq_halves<<<grid_for(J.begin[J.count], 256), 256, 0, g->ctx->stream>>>(J);
-    VG_LAUNCHED(g->ctx);
-    return VG_OK;
-}
-
-static int build_halves(vg_gkr *g, const fe *r_dev, int len, fe scale, fe *lo, fe *hi, int *fh)
-{
-    EqJobs J{};
-    add_halves(J, r_dev, len, scale, lo, hi, fh);
-    return launch_halves(g, J);
-}
-
-static int upload_r(vg_gkr *g, int slot, const vg_fe *r, int len)
-{
-    if (len > 64) return vg_fail(VG_ERR_ARG, "challenge vector longer than 64");
-    if (len == 0) return VG_OK;
-    VG_CHECK_CUDA(cudaMemcpyAsync(g->rbuf + 64 * slot, r, len * sizeof(fe), cudaMemcpyHostToDevice, g->ctx->stream));
+    k_eq_halves<<<grid_for(J.begin[J.count] + 1, 128), 128, 0, c->stream>>>(J);
+    VG_LAUNCHED(c);
     return VG_OK;
 }
 
@@ -2194,10 +2174,11 @@ extern "C" int vg_gkr_v_res(vg_gkr *g, const vg_fe *r, int r_len, vg_fe *out)
     if (r_len != g->C->L[last].bl) return vg_fail(VG_ERR_ARG, "r_len %d != output bit length %d", r_len, g->C->L[last].bl);
     vg_ctx *c = g->ctx;
     VG_TRY(flush_rounds(g));
-    VG_TRY(upload_r(g, 0, r, r_len));
     fe *lo = g->eq, *hi = g->eq + g->eq_half;
     int fh;
-    VG_TRY(build_halves(g, g->rbuf, r_len, vg::fe_one(), lo, hi, &fh));
+    EqJobs J{};
+    add_halves(J, r, r_len, vg::fe_one(), lo, hi, &fh);
+    VG_TRY(launch_halves(c, J));
     fe *parts;
     const int nb = 148 * 2;
     VG_TRY(vg_partials(c, nb + 1, &parts));
@@ -2254,15 +2235,14 @@ extern "C" int vg_mle_eval(vg_ctx *c, const vg_fe *vals, long n, const vg_fe *r,
 static int eq_table(vg_ctx *c, const vg_fe *r, int log_len, vg_fe *pub)
 {
     if (!c || !r || !pub || log_len < 1 || log_len > 30) return vg_fail(VG_ERR_ARG, "vg_eq_table: bad argument");
-    fe *tmp;
-    int f = log_len >> 1, s = log_len - f;
-    VG_TRY(vg_scratch2(c, ((1L << f) + (1L << s) + 64) * sizeof(fe), (void **)&tmp));
-    fe *lo = tmp, *hi = tmp + (1L << f), *rd = hi + (1L << s);
-    VG_CHECK_CUDA(cudaMemcpyAsync(rd, r, log_len * sizeof(fe), cudaMemcpyHostToDevice, c->stream));   // staged copy
-    k_eq_half<<<grid_for(1L << f, 256), 256, 0, c->stream>>>(rd, f, vg::fe_one(), lo);
-    c->launches++;
-    k_eq_half<<<grid_for(1L << s, 256), 256, 0, c->stream>>>(rd + f, s, vg::fe_one(), hi);
-    c->launches++;
+    fe *lo;
+    const int s = log_len - (log_len >> 1);
+    VG_TRY(vg_scratch2(c, (2L << s) * sizeof(fe), (void **)&lo));
+    fe *hi = lo + (1L << s);
+    int f;
+    EqJobs J{};
+    add_halves(J, r, log_len, vg::fe_one(), lo, hi, &f);
+    VG_TRY(launch_halves(c, J));
     long n = 1L << log_len;
     k_eq_combine<<<std::min<unsigned>(grid_for(n, 256), 148u * 32u), 256, 0, c->stream>>>(lo, hi, f, n, (fe *)pub);
     VG_LAUNCHED(c);
@@ -2292,26 +2272,20 @@ extern "C" int vg_circuit_predicates(vg_ctx *c, const vg_circuit *C, int layer, 
     const int fg = lg >> 1, sg = lg - fg, fuv = luv >> 1, suv = luv - fuv;
     const long hg = 1L << std::max(fg, sg), huv = 1L << std::max(fuv, suv);
     const int nb = 148 * 4;
-    // scratch: r values, 4 g halves, 4 u/v halves, partials, result
-    const size_t n_fe = 4 * 64 + 4 * hg + 4 * huv + (size_t)nb * 14 + 16;
+    // scratch: 4 g halves, 4 u/v halves, partials, result
+    const size_t n_fe = 4 * hg + 4 * huv + (size_t)nb * 14 + 16;
     fe *w;
     VG_TRY(vg_scratch(c, n_fe * sizeof(fe), (void **)&w));
-    fe *rr = w, *tg = rr + 4 * 64, *tuv = tg + 4 * hg, *parts = tuv + 4 * huv, *res = parts + (size_t)nb * 14;
-    VG_CHECK_CUDA(cudaMemcpyAsync(rr, r_0, lg * sizeof(fe), cudaMemcpyHostToDevice, c->stream));
-    VG_CHECK_CUDA(cudaMemcpyAsync(rr + 64, r_1, lg * sizeof(fe), cudaMemcpyHostToDevice, c->stream));
-    VG_CHECK_CUDA(cudaMemcpyAsync(rr + 128, r_u, luv * sizeof(fe), cudaMemcpyHostToDevice, c->stream));
-    VG_CHECK_CUDA(cudaMemcpyAsync(rr + 192, r_v, luv * sizeof(fe), cudaMemcpyHostToDevice, c->stream));
+    fe *tg = w, *tuv = tg + 4 * hg, *parts = tuv + 4 * huv, *res = parts + (size_t)nb * 14;
     int fh;
     EqJobs J1{}, J2{};
-    add_halves(J1, rr, lg, tofe(alpha), tg, tg + hg, &fh);
-    add_halves(J1, rr + 64, lg, tofe(beta), tg + 2 * hg, tg + 3 * hg, &fh);
-    add_halves(J2, rr + 128, luv, vg::fe_one(), tuv, tuv + huv, &fh);
-    add_halves(J2, rr + 192, luv, vg::fe_one(), tuv + 2 * huv, tuv + 3 * huv, &fh);
-    for (const EqJobs *J : {&J1, &J2}) {
-        k_eq_halves<<<grid_for(J->begin[J->count], 256), 256, 0, c->stream>>>(*J);
-        VG_LAUNCHED(c);
-    }
-    BetaG bg{tg, tg + hg, tg + 2 * hg, tg + 3 * hg, fg, (1L << fg) - 1};
+    add_halves(J1, r_0, lg, tofe(alpha), tg, tg + 2 * hg, &fh, 2);
+    add_halves(J1, r_1, lg, tofe(beta), tg + 1, tg + 2 * hg + 1, &fh, 2);
+    add_halves(J2, r_u, luv, vg::fe_one(), tuv, tuv + huv, &fh);
+    add_halves(J2, r_v, luv, vg::fe_one(), tuv + 2 * huv, tuv + 3 * huv, &fh);
+    VG_TRY(launch_halves(c, J1));
+    VG_TRY(launch_halves(c, J2));
+    BetaG bg{tg, tg + 2 * hg, fg, (1L << fg) - 1};
     BetaU bu{tuv, tuv + huv, fuv, (1L << fuv) - 1};
     BetaU bv{tuv + 2 * huv, tuv + 3 * huv, fuv, (1L << fuv) - 1};
     k_predicates<<<nb, PRED_THREADS, 0, c->stream>>>(D.ty, D.u, D.v, D.n, bg, bu, bv, (uint32_t)((1L << luv) - 1), parts);
@@ -2433,21 +2407,17 @@ extern "C" int vg_gkr_phase1_init(vg_gkr *g, int layer, const vg_fe *r0, const v
     const long N = g->C->L[layer - 1].n, maxN = 1L << g->C->max_bl;
     g->layer = layer;
     g->length_g = length_g;
-    VG_TRY(upload_r(g, 0, r0, length_g));
-    VG_TRY(upload_r(g, 1, r1, length_g));
     fe *e = g->eq;
     const long H = g->eq_half;
     int fh;
     {   // the alpha- and beta-weighted tables of r0 and r1 in one launch
         EqJobs J{};
-        add_halves(J, g->rbuf, length_g, tofe(alpha), e, e + H, &fh);
-        add_halves(J, g->rbuf + 64, length_g, tofe(beta), e + 2 * H, e + 3 * H, &fh);
-        VG_TRY(launch_halves(g, J));
+        add_halves(J, r0, length_g, tofe(alpha), e, e + 2 * H, &fh, 2);
+        add_halves(J, r1, length_g, tofe(beta), e + 1, e + 2 * H + 1, &fh, 2);
+        VG_TRY(launch_halves(c, J));
     }
-    g->bg.f0 = e;
-    g->bg.s0 = e + H;
-    g->bg.f1 = e + 2 * H;
-    g->bg.s1 = e + 3 * H;
+    g->bg.f = e;
+    g->bg.s = e + 2 * H;
     g->bg.fh = fh;
     g->bg.mask = (1L << fh) - 1;
     g->bg.save = nullptr;
@@ -2705,7 +2675,7 @@ static int exec_pending(vg_gkr *g)
         key.push_back((uint64_t)L.G.slot0);
         if (L.kind == 3) {
             const GatherArgs &a = L.ga;
-            const void *ptrs[] = {a.e.off, a.e.g, a.e.o, a.e.tk, a.bg.f0, a.bg.s0, a.bg.f1, a.bg.s1, a.bg.save,
+            const void *ptrs[] = {a.e.off, a.e.g, a.e.o, a.e.tk, a.bg.f, a.bg.s, a.bg.save,
                                   a.bg.tab, a.bu.f, a.bu.s, a.prev, a.vu, a.tm, a.tv};
             for (const void *q : ptrs) key.push_back((uint64_t)(uintptr_t)q);
             key.push_back((uint64_t)(uint32_t)a.bg.fh | ((uint64_t)(uint32_t)a.bu.fh << 16) | ((uint64_t)L.ph << 32));
@@ -2899,17 +2869,17 @@ static int flush_rounds(vg_gkr *g)
     return exec_pending(g);
 }
 
-// phase-2 tables for the current layer once g->vu holds v_u
-static int phase2_tables(vg_gkr *g, const vg_fe *r_u, int length_u)
+// phase-2 tables for the current layer; J: how v_u is formed, if the host has not set it
+static int phase2_tables(vg_gkr *g, const vg_fe *r_u, int length_u, EqJobs &J)
 {
     const int layer = g->layer;
     vg_ctx *c = g->ctx;
     const DevLayer &D = g->C->L[layer];
     const long N = g->C->L[layer - 1].n, maxN = 1L << g->C->max_bl;
-    VG_TRY(upload_r(g, 2, r_u, length_u));
     fe *e = g->eq + 4 * g->eq_half;
     int fh;
-    VG_TRY(build_halves(g, g->rbuf + 128, length_u, vg::fe_one(), e, e + g->eq_half, &fh));
+    add_halves(J, r_u, length_u, vg::fe_one(), e, e + g->eq_half, &fh);
+    VG_TRY(launch_halves(c, J));
     BetaU bu;
     bu.f = e;
     bu.s = e + g->eq_half;
@@ -2952,7 +2922,8 @@ extern "C" int vg_gkr_phase2_init(vg_gkr *g, const vg_fe *r_u, int length_u, vg_
     VG_TRY(phase2_check(g, r_u, length_u));
     fe vu = tofe(v_u);
     VG_CHECK_CUDA(cudaMemcpyAsync(g->vu, &vu, sizeof(fe), cudaMemcpyHostToDevice, g->ctx->stream));   // staged copy
-    return phase2_tables(g, r_u, length_u);
+    EqJobs J{};
+    return phase2_tables(g, r_u, length_u, J);
 }
 
 int vg_gkr_phase2_init_deferred(vg_gkr *g, const vg_fe *r_u, int length_u, vg_fe r_last, vg_fe addend)
@@ -2960,9 +2931,12 @@ int vg_gkr_phase2_init_deferred(vg_gkr *g, const vg_fe *r_u, int length_u, vg_fe
     VG_TRY(phase2_check(g, r_u, length_u));
     if (!g->deferred || g->rec_n < 1 || g->n != 2)
         return vg_fail(VG_ERR_STATE, "deferred phase2_init must follow the last deferred phase-1 round");
-    k_vu<<<1, 1, 0, g->ctx->stream>>>(g->rec + 9 * (g->rec_n - 1) + 3, tofe(r_last), tofe(addend), g->vu);
-    VG_LAUNCHED(g->ctx);
-    return phase2_tables(g, r_u, length_u);
+    EqJobs J{};
+    J.last6 = g->rec + 9 * (g->rec_n - 1) + 3;
+    J.vu_r = tofe(r_last);
+    J.vu_add = tofe(addend);
+    J.vu = g->vu;
+    return phase2_tables(g, r_u, length_u, J);
 }
 
 // challenge slots for n records: device copy from the pool, pinned host side
