@@ -52,9 +52,11 @@ struct vg_ctx {
     fe *pinned = nullptr;    // pinned host staging for small results
     size_t pinned_cap = 0;
     // pinned ring for uploads from pageable host memory (vg_h2d_staged)
-    char *ring[2] = {nullptr, nullptr};
+    static constexpr int RING = 4;
+    char *ring = nullptr;    // RING chunks, ring_next the one to fill next
+    int ring_next = 0;
     std::vector<void *> retired_pinned;   // outgrown pinned blocks, freed with the context
-    cudaEvent_t ring_ev[2] = {nullptr, nullptr};
+    cudaEvent_t ring_ev[RING] = {};
     // per-launch profiler: event pairs around launches of each kernel family
     bool profiling = false;
     std::vector<ProfRec> prof;
@@ -113,9 +115,9 @@ int vg_fail(int code, const char *fmt, ...);
     } while (0)
 
 // Host-to-device copy on the context stream.  Pageable sources go through the
-// context's two pinned chunks (host memcpy of one chunk overlaps the DMA of
-// the other), so concurrent sessions do not serialise on the driver's
-// staging.  A pageable source may be reused on return; a pinned or device
+// context's ring of pinned chunks (the host copies one while those before it
+// are on their way, across calls as well), so concurrent sessions do not
+// serialise on the driver's staging.  A pageable source may be reused on return; a pinned or device
 // source is copied directly and must stay valid until the stream reaches the
 // copy.
 int vg_h2d_staged(vg_ctx *c, void *dst, const void *src, size_t bytes);
@@ -258,11 +260,6 @@ __device__ __forceinline__ bool grid_sum(const fe (&acc)[K], uint32_t (&sw)[16][
 
 // sum of `nparts` groups of K partials (layout [part][K]) into out[K]
 int vg_reduce_partials(vg_ctx *ctx, const fe *parts, int nparts, int K, fe *out_dev);
-
-// Exclusive prefix sum of d[0 .. n) in place, d[n] (zero on entry) receives
-// the total; tmp holds vg_scan_tmp_words(n) words.
-long vg_scan_tmp_words(long n);
-int vg_scan_u32(vg_ctx *c, uint32_t *d, long n, uint32_t *tmp);
 
 // The device's launch-shape parameter `key` (VG_TUNE_*; tune.cu).
 long vg_tune_value(int device, int key);

@@ -64,7 +64,8 @@ struct DevLayer {
 
 constexpr int LIGHT_MAX = 64;   // edges a single thread sums; longer lists get a warp
 constexpr long HEAVY_MIN = 32768;   // longer lists are split over many CTAs
-constexpr int EDGE_STATS = 4;       // per edge set: total, long keys, overflow, heavy keys
+constexpr int HEAVY_INLINE = 8;     // heavy keys that travel with a set's counts
+constexpr int EDGE_STATS = 4 + (3 * HEAVY_INLINE + 1) / 2;   // per edge set: total, long keys, overflow, heavy keys, the first of them
 constexpr int MAX_HEAVY = 16;       // heavy keys per launch
 constexpr int HEAVY_PARTS = 296;    // CTAs per heavy key
 
@@ -433,76 +434,213 @@ __global__ void __launch_bounds__(GKR_THREADS) k_phase2_scatter(const uint8_t *_
 }
 
 // ------------------------------------------------------- wiring transpose
-// Calls emit(key, gate, other, type | doublings << 8) for every edge of gate
-// g in phase PH (0: keyed by u as in k_phase1_scatter, 1: keyed by v as in
-// k_phase2_scatter, summation gates at key 0).
-template <int PH, typename Emit>
-__device__ __forceinline__ void gate_edges(int t, uint32_t g, uint32_t u, uint32_t v, Emit emit)
+// The wires of both phases' edge sets, three launches for a layer: keys are
+// counted, the counts become offsets, cursors and lists of long keys, and the
+// edges are placed.  Each launch covers both phases (a gate's type and wires
+// are read once for the two), so a layer takes five enqueues with its memset
+// where a set of its own for each phase, with a general scan, took eighteen:
+// builds of many small layers are bound by the enqueues, and the edge sets of
+// a 2^22-gate circuit of 16 layers and of a SHA-256 circuit's 10 layers took
+// 1.3 and 1.55 ms of a load.
+struct EdgeOut {
+    uint32_t *cur;             // counts, then cursors (N)
+    uint32_t *off;             // N + 1
+    uint32_t *g, *o;
+    uint16_t *tk;
+    uint32_t *list, *heavy;    // keys with more than LIGHT_MAX edges; (key, first, end) beyond HEAVY_MIN
+    long cap, cap_list, cap_heavy;
+    unsigned long long *st;    // EDGE_STATS words
+};
+struct EdgeBuild {
+    EdgeOut ph[2];
+};
+
+// Calls run(key, step, n, gate, other, ostep, type | doublings << 8, dstep) for
+// the edges of gate g in phase PH (0: keyed by u as in k_phase1_scatter, 1:
+// keyed by v as in k_phase2_scatter, summation gates at key 0): edge j < n has
+// key + j step, other + j ostep and the last argument + j dstep.
+template <int PH, typename Run>
+__device__ __forceinline__ void gate_edges(int t, uint32_t g, uint32_t u, uint32_t v, Run run)
 {
     if (t == 2 || t == 3 || t == 11 || t > 13) return;
     if (PH == 0) {
-        if (t == 4) emit(u, u, 0u, (uint16_t)4);
-        else if (t == 5)
-            for (uint32_t j = u; j < v; ++j) emit(j, g, 0u, (uint16_t)5);
-        else if (t == 12)
-            for (uint32_t j = u; j <= v; ++j) emit(j, g, 0u, (uint16_t)(12 | ((j - u) << 8)));
-        else emit(u, g, v, (uint16_t)t);
+        if (t == 4) run(u, 0u, 1u, u, 0u, 0u, 4u, 0u);
+        else if (t == 5) run(u, 1u, v > u ? v - u : 0u, g, 0u, 0u, 5u, 0u);
+        else if (t == 12) run(u, 1u, v >= u ? v - u + 1 : 0u, g, 0u, 0u, 12u, 1u << 8);
+        else run(u, 0u, 1u, g, v, 0u, (uint32_t)t, 0u);
     } else {
         if (t == 4) return;
-        if (t == 5)
-            for (uint32_t j = u; j < v; ++j) emit(0u, g, j, (uint16_t)5);
-        else if (t == 12)
-            for (uint32_t j = u; j <= v; ++j) emit(0u, g, j, (uint16_t)(12 | ((j - u) << 8)));
-        else emit(v, g, u, (uint16_t)t);
+        if (t == 5) run(0u, 0u, v > u ? v - u : 0u, g, u, 1u, 5u, 0u);
+        else if (t == 12) run(0u, 0u, v >= u ? v - u + 1 : 0u, g, u, 1u, 12u, 1u << 8);
+        else run(v, 0u, 1u, g, u, 0u, (uint32_t)t, 0u);
     }
 }
 
-// FILL == false: count edges per key; FILL == true: place them (cursor holds
-// the offsets on entry) unless the total exceeds cap, which sets stats[2].
+// Edges of each key, and each set's total (st[0], 64 bits wide: sums of wide
+// ranges can pass 2^32).  Edges of one gate at one key are one atomic.
+template <int PH>
+__device__ __forceinline__ unsigned long long count_gate(int t, uint32_t g, uint32_t u, uint32_t v, uint32_t *cnt)
+{
+    unsigned long long total = 0;
+    gate_edges<PH>(t, g, u, v, [&](uint32_t key, uint32_t step, uint32_t n, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t) {
+        total = n;
+        if (!step) {
+            if (n) atomicAdd(&cnt[key], n);
+        } else
+            for (uint32_t j = 0; j < n; ++j) atomicAdd(&cnt[key + j], 1u);
+    });
+    return total;
+}
+__global__ void __launch_bounds__(GKR_THREADS) k_edge_counts(const uint8_t *__restrict__ ty, const uint32_t *__restrict__ uu,
+                                                             const uint32_t *__restrict__ vv, long ng,
+                                                             const __grid_constant__ EdgeBuild B)
+{
+    unsigned long long t0 = 0, t1 = 0;
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < ng; i += (long)gridDim.x * blockDim.x) {
+        const int t = ty[i];
+        const uint32_t u = uu[i], v = vv[i];
+        t0 += count_gate<0>(t, (uint32_t)i, u, v, B.ph[0].cur);
+        t1 += count_gate<1>(t, (uint32_t)i, u, v, B.ph[1].cur);
+    }
+    for (int d = 16; d; d >>= 1) {
+        t0 += __shfl_xor_sync(0xffffffffu, t0, d);
+        t1 += __shfl_xor_sync(0xffffffffu, t1, d);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (t0) atomicAdd(&B.ph[0].st[0], t0);
+        if (t1) atomicAdd(&B.ph[1].st[0], t1);
+    }
+}
+
+// Exclusive prefix of x over the CTA's threads, and the CTA's sum.
+__device__ __forceinline__ uint32_t cta_prefix(uint32_t x, uint32_t *sm, uint32_t &sum)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t incl = x;
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += y;
+    }
+    __syncthreads();   // sm is free again
+    if (lane == 31) sm[w] = incl;
+    __syncthreads();
+    uint32_t below = 0;
+    sum = 0;
+    for (int q = 0; q < GKR_THREADS / 32; ++q) {
+        const uint32_t y = sm[q];
+        below += q < w ? y : 0u;
+        sum += y;
+    }
+    return below + incl - x;
+}
+
+// CTA (b, ph) owns keys [b span, (b + 1) span): the first launch sums their
+// counts, the second adds the sums of the spans before its own (there are at
+// most EDGE_SPANS, so no scan of the sums is needed) and turns its counts into
+// offsets.  A thread takes OFF_PER neighbouring keys of each tile.
+constexpr int EDGE_SPANS = 1024, OFF_PER = 8;
+constexpr long OFF_TILE = (long)GKR_THREADS * OFF_PER;
+
+__global__ void __launch_bounds__(GKR_THREADS) k_edge_spans(const __grid_constant__ EdgeBuild B, long N, long span,
+                                                            uint32_t *__restrict__ sums)
+{
+    __shared__ uint32_t sm[GKR_THREADS / 32];
+    const uint32_t *cnt = B.ph[blockIdx.y].cur;
+    const long lo = blockIdx.x * span, hi = min(N, lo + span);
+    uint32_t x = 0, sum;
+    for (long k = lo + threadIdx.x; k < hi; k += GKR_THREADS) x += cnt[k];
+    cta_prefix(x, sm, sum);
+    if (threadIdx.x == 0) sums[blockIdx.y * EDGE_SPANS + blockIdx.x] = sum;
+}
+
+// Offsets, cursors, the list of keys with more than LIGHT_MAX edges (st[1] of
+// them) and the keys with more than HEAVY_MIN (st[3]; the first HEAVY_INLINE
+// triples also in st).  A list takes one atomic per tile and keeps the keys of
+// a tile in order, so the warps that sum them write neighbouring entries.
+__global__ void __launch_bounds__(GKR_THREADS) k_edge_offsets(const __grid_constant__ EdgeBuild B, long N, long span,
+                                                              const uint32_t *__restrict__ sums)
+{
+    __shared__ uint32_t sm[GKR_THREADS / 32];
+    __shared__ unsigned long long first;
+    const EdgeOut &E = B.ph[blockIdx.y];
+    const long lo = blockIdx.x * span, hi = min(N, lo + span);
+    uint32_t base = 0, x = 0, sum;
+    for (int b = threadIdx.x; b < (int)blockIdx.x; b += GKR_THREADS) x += sums[blockIdx.y * EDGE_SPANS + b];
+    cta_prefix(x, sm, base);
+    for (long t0 = lo; t0 < hi; t0 += OFF_TILE) {
+        const long k0 = t0 + (long)threadIdx.x * OFF_PER;
+        uint32_t c[OFF_PER], n_long = 0;
+        x = 0;
+#pragma unroll
+        for (int j = 0; j < OFF_PER; ++j) {
+            c[j] = k0 + j < hi ? E.cur[k0 + j] : 0u;
+            x += c[j];
+            n_long += c[j] > (uint32_t)LIGHT_MAX && c[j] <= (uint32_t)HEAVY_MIN;
+        }
+        uint32_t p = base + cta_prefix(x, sm, sum);
+        base += sum;
+#pragma unroll
+        for (int j = 0; j < OFF_PER; ++j) {
+            if (k0 + j >= hi) break;
+            E.off[k0 + j] = p;
+            E.cur[k0 + j] = p;
+            if (c[j] > (uint32_t)HEAVY_MIN) {
+                const unsigned long long i = atomicAdd(&E.st[3], 1ull);
+                const uint32_t tri[3] = {(uint32_t)(k0 + j), p, p + c[j]};
+                for (int q = 0; q < 3; ++q) {
+                    if ((long)i < E.cap_heavy) E.heavy[3 * i + q] = tri[q];
+                    if (i < (unsigned long long)HEAVY_INLINE) ((uint32_t *)(E.st + 4))[3 * i + q] = tri[q];
+                }
+            }
+            p += c[j];
+        }
+        if (__syncthreads_or(n_long != 0)) {
+            uint32_t q = cta_prefix(n_long, sm, sum);
+            if (threadIdx.x == 0) first = atomicAdd(&E.st[1], (unsigned long long)sum);
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < OFF_PER; ++j)
+                if (c[j] > (uint32_t)LIGHT_MAX && c[j] <= (uint32_t)HEAVY_MIN) {
+                    if ((long)(first + q) < E.cap_list) E.list[first + q] = (uint32_t)(k0 + j);
+                    ++q;
+                }
+        }
+    }
+    if (hi == N && threadIdx.x == 0) E.off[N] = base;
+}
+
+// Places the edges unless a set's total exceeds its room, which sets st[2].
 // The order inside a key is not fixed, which does not matter: the gathers sum
 // exactly in F_p2.
-template <int PH, bool FILL>
-__global__ void k_edges(const uint8_t *__restrict__ ty, const uint32_t *__restrict__ uu, const uint32_t *__restrict__ vv,
-                        long ng, uint32_t *__restrict__ cnt, uint32_t *__restrict__ eg, uint32_t *__restrict__ eo,
-                        uint16_t *__restrict__ etk, const uint32_t *__restrict__ total, long cap,
-                        unsigned long long *__restrict__ stats)
+template <int PH>
+__device__ __forceinline__ void place_gate(int t, uint32_t g, uint32_t u, uint32_t v, const EdgeOut &E)
 {
-    if (FILL && (long)*total > cap) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) stats[2] = 1;
-        return;
+    gate_edges<PH>(t, g, u, v, [&](uint32_t key, uint32_t step, uint32_t n, uint32_t gv, uint32_t o, uint32_t ostep,
+                                   uint32_t tk, uint32_t dstep) {
+        uint32_t p = 0;
+        if (!step && n) p = atomicAdd(&E.cur[key], n);
+        for (uint32_t j = 0; j < n; ++j) {
+            if (step) p = atomicAdd(&E.cur[key + j], 1u) - j;
+            E.g[p + j] = gv;
+            E.o[p + j] = o + j * ostep;
+            E.tk[p + j] = (uint16_t)(tk + j * dstep);
+        }
+    });
+}
+__global__ void __launch_bounds__(GKR_THREADS) k_edge_fill(const uint8_t *__restrict__ ty, const uint32_t *__restrict__ uu,
+                                                           const uint32_t *__restrict__ vv, long ng,
+                                                           const __grid_constant__ EdgeBuild B)
+{
+    bool fits[2];
+    for (int q = 0; q < 2; ++q) {
+        fits[q] = B.ph[q].st[0] <= (unsigned long long)B.ph[q].cap;
+        if (!fits[q] && blockIdx.x == 0 && threadIdx.x == 0) B.ph[q].st[2] = 1;
     }
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < ng; i += (long)gridDim.x * blockDim.x) {
-        gate_edges<PH>(ty[i], (uint32_t)i, uu[i], vv[i], [&](uint32_t key, uint32_t gv, uint32_t o, uint16_t tk) {
-            const uint32_t p = atomicAdd(&cnt[key], 1u);
-            if (FILL) {
-                eg[p] = gv;
-                eo[p] = o;
-                etk[p] = tk;
-            }
-        });
-    }
-}
-
-// keys with more than LIGHT_MAX edges into list (room for cap_list), those
-// with more than HEAVY_MIN as (key, first, end) triples into heavy;
-// stats[0] = edge total, stats[1] = listed keys, stats[3] = heavy keys
-__global__ void k_medium_keys(const uint32_t *__restrict__ off, long N, uint32_t *__restrict__ list, long cap_list,
-                              uint32_t *__restrict__ heavy, long cap_heavy, unsigned long long *__restrict__ stats)
-{
-    if (blockIdx.x == 0 && threadIdx.x == 0) stats[0] = off[N];
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < N; k += (long)gridDim.x * blockDim.x) {
-        const uint32_t len = off[k + 1] - off[k];
-        if (len > (uint32_t)HEAVY_MIN) {
-            const unsigned long long i = atomicAdd(&stats[3], 1ull);
-            if ((long)i < cap_heavy) {
-                heavy[3 * i] = (uint32_t)k;
-                heavy[3 * i + 1] = off[k];
-                heavy[3 * i + 2] = off[k + 1];
-            }
-        } else if (len > (uint32_t)LIGHT_MAX) {
-            const unsigned long long i = atomicAdd(&stats[1], 1ull);
-            if ((long)i < cap_list) list[i] = (uint32_t)k;
-        }
+        const int t = ty[i];
+        const uint32_t u = uu[i], v = vv[i];
+        if (fits[0]) place_gate<0>(t, (uint32_t)i, u, v, B.ph[0]);
+        if (fits[1]) place_gate<1>(t, (uint32_t)i, u, v, B.ph[1]);
     }
 }
 
@@ -1415,9 +1553,9 @@ struct vg_circuit {
     void *staging = nullptr;   // upload staging for one layer
     size_t staging_cap = 0;
     unsigned long long *err = nullptr;
-    uint32_t *work = nullptr;   // edge build: cursors and scan temporaries
+    uint32_t *work = nullptr;   // edge build: both phases' cursors and span sums
     size_t work_cap = 0;        // words
-    unsigned long long *edge_stats = nullptr;   // 3 per edge set: total, long keys, overflow
+    unsigned long long *edge_stats = nullptr;   // EDGE_STATS per edge set
     int edge_stats_cap = 0;
     std::vector<unsigned long long> edge_stats_host;
 };
@@ -1554,35 +1692,10 @@ static int alloc_edges(vg_ctx *c, EdgeSet &E, long n)
     return VG_OK;
 }
 
-// Enqueues the fill of edge set ph of layer li (offsets already scanned) and
-// the list of its long keys.
-static int fill_edges(vg_circuit *c, int li, int ph)
-{
-    vg_ctx *ctx = c->ctx;
-    DevLayer &D = c->L[li];
-    EdgeSet &E = D.ph[ph];
-    const long N = E.N;
-    unsigned long long *st = c->edge_stats + EDGE_STATS * (2 * li + ph);
-    const unsigned grid = std::min<unsigned>(grid_for(D.n, 256), 148u * 32u);
-    VG_CHECK_CUDA(cudaMemsetAsync(st, 0, EDGE_STATS * 8, ctx->stream));
-    VG_CHECK_CUDA(cudaMemcpyAsync(c->work, E.off, N * 4, cudaMemcpyDeviceToDevice, ctx->stream));
-    if (ph == 0)
-        k_edges<0, true><<<grid, 256, 0, ctx->stream>>>(D.ty, D.u, D.v, D.n, c->work, E.g, E.o, E.tk, E.off + N, E.cap_E, st);
-    else
-        k_edges<1, true><<<grid, 256, 0, ctx->stream>>>(D.ty, D.u, D.v, D.n, c->work, E.g, E.o, E.tk, E.off + N, E.cap_E, st);
-    VG_LAUNCHED(ctx);
-    // a key with more than LIGHT_MAX edges: at most cap_E / (LIGHT_MAX + 1) of them
-    VG_TRY(grow_u32(ctx, &E.medium, &E.cap_M, E.cap_E / (LIGHT_MAX + 1) + 1));
-    VG_TRY(grow_u32(ctx, &E.heavy, &E.cap_H, 3 * (E.cap_E / HEAVY_MIN + 1)));
-    k_medium_keys<<<std::min<unsigned>(grid_for(N, 256), 148u * 32u), 256, 0, ctx->stream>>>(
-        E.off, N, E.medium, E.cap_M, E.heavy, E.cap_H / 3, st);
-    VG_LAUNCHED(ctx);
-    return VG_OK;
-}
-
 // Enqueues the phase-1 and phase-2 edge sets of prover layer li (see
 // EdgeSet), without synchronising: the edge arrays are sized for one edge per
-// gate, and a set that needs more is rebuilt by finish_edges.
+// gate, and a set that needs more is rebuilt by finish_edges.  The layer's
+// counts are zero on entry (start_edges).
 static int launch_edges(vg_circuit *c, int li)
 {
     vg_ctx *ctx = c->ctx;
@@ -1592,8 +1705,7 @@ static int launch_edges(vg_circuit *c, int li)
     const char *mode = getenv("VIRGO_PHASE_TABLES");   // "atomic": keep the scatter path (tests compare both)
     if (mode && !strcmp(mode, "atomic")) return VG_OK;
     const long N = c->L[li - 1].n;
-    const unsigned grid = std::min<unsigned>(grid_for(D.n, 256), 148u * 32u);
-    const size_t work = (size_t)N + (size_t)vg_scan_tmp_words(N);
+    const size_t work = 2 * (size_t)N + 2 * EDGE_SPANS;
     if (work > c->work_cap) {
         vg_release(ctx, c->work);
         c->work = nullptr;
@@ -1601,29 +1713,38 @@ static int launch_edges(vg_circuit *c, int li)
         VG_TRY(vg_alloc(ctx, (void **)&c->work, work * 4));
         c->work_cap = work;
     }
+    EdgeBuild B;
     for (int ph = 0; ph < 2; ++ph) {
         EdgeSet &E = D.ph[ph];
         E.N = N;
         VG_TRY(grow_u32(ctx, &E.off, &E.cap_N, N + 1));
         if (E.cap_E < D.n) VG_TRY(alloc_edges(ctx, E, D.n));
-        VG_CHECK_CUDA(cudaMemsetAsync(E.off, 0, (N + 1) * 4, ctx->stream));
-        if (ph == 0)
-            k_edges<0, false><<<grid, 256, 0, ctx->stream>>>(D.ty, D.u, D.v, D.n, E.off, nullptr, nullptr, nullptr, nullptr, 0,
-                                                            nullptr);
-        else
-            k_edges<1, false><<<grid, 256, 0, ctx->stream>>>(D.ty, D.u, D.v, D.n, E.off, nullptr, nullptr, nullptr, nullptr, 0,
-                                                            nullptr);
-        VG_LAUNCHED(ctx);
-        VG_TRY(vg_scan_u32(ctx, E.off, N, c->work + N));
-        VG_TRY(fill_edges(c, li, ph));
-        E.launched = true;
+        // a key with more than LIGHT_MAX edges: at most cap_E / (LIGHT_MAX + 1) of them
+        VG_TRY(grow_u32(ctx, &E.medium, &E.cap_M, E.cap_E / (LIGHT_MAX + 1) + 1));
+        VG_TRY(grow_u32(ctx, &E.heavy, &E.cap_H, 3 * (E.cap_E / HEAVY_MIN + 1)));
+        B.ph[ph] = {c->work + ph * N, E.off, E.g, E.o, E.tk, E.medium, E.heavy, E.cap_E, E.cap_M, E.cap_H / 3,
+                    c->edge_stats + EDGE_STATS * (2 * li + ph)};
     }
+    const long span = OFF_TILE * ((N + OFF_TILE * EDGE_SPANS - 1) / (OFF_TILE * EDGE_SPANS));
+    const dim3 spans((unsigned)((N + span - 1) / span), 2);
+    uint32_t *sums = c->work + 2 * N;
+    const unsigned grid = std::min<unsigned>(grid_for(D.n, GKR_THREADS), 148u * 32u);
+    VG_CHECK_CUDA(cudaMemsetAsync(c->work, 0, 2 * (size_t)N * 4, ctx->stream));
+    k_edge_counts<<<grid, GKR_THREADS, 0, ctx->stream>>>(D.ty, D.u, D.v, D.n, B);
+    VG_LAUNCHED(ctx);
+    k_edge_spans<<<spans, GKR_THREADS, 0, ctx->stream>>>(B, N, span, sums);
+    VG_LAUNCHED(ctx);
+    k_edge_offsets<<<spans, GKR_THREADS, 0, ctx->stream>>>(B, N, span, sums);
+    VG_LAUNCHED(ctx);
+    k_edge_fill<<<grid, GKR_THREADS, 0, ctx->stream>>>(D.ty, D.u, D.v, D.n, B);
+    VG_LAUNCHED(ctx);
+    D.ph[0].launched = D.ph[1].launched = true;
     return VG_OK;
 }
 
-// Enqueues the edge sets of every layer and the copy of their counts to
-// c->edge_stats_host (valid after the stream is synchronised).
-static int launch_all_edges(vg_circuit *c)
+// Room for every layer's edge counts, zeroed; launch_edges may follow layer by
+// layer, while later layers are still on their way to the device.
+static int start_edges(vg_circuit *c)
 {
     const int need = EDGE_STATS * 2 * c->depth;
     if (need > c->edge_stats_cap) {
@@ -1635,63 +1756,68 @@ static int launch_all_edges(vg_circuit *c)
     }
     c->edge_stats_host.assign(need, 0);
     VG_CHECK_CUDA(cudaMemsetAsync(c->edge_stats, 0, need * 8, c->ctx->stream));
-    for (int li = 1; li < c->depth; ++li) VG_TRY(launch_edges(c, li));
-    VG_CHECK_CUDA(cudaMemcpyAsync(c->edge_stats_host.data(), c->edge_stats, need * 8, cudaMemcpyDeviceToHost, c->ctx->stream));
     return VG_OK;
 }
 
-// The heavy keys' (key, first, end) triples to the host (circuits that have
-// any: one more synchronisation at build time).
-static int read_heavy(vg_circuit *c, EdgeSet &E, long n_heavy)
+// The counts to c->edge_stats_host, and the stream synchronised.
+static int read_edge_stats(vg_circuit *c)
 {
+    VG_CHECK_CUDA(cudaMemcpyAsync(c->edge_stats_host.data(), c->edge_stats, EDGE_STATS * 2 * (size_t)c->depth * 8,
+                                  cudaMemcpyDeviceToHost, c->ctx->stream));
+    VG_CHECK_CUDA(cudaStreamSynchronize(c->ctx->stream));
+    return VG_OK;
+}
+
+// The heavy keys' (key, first, end) triples to the host: the first ones came
+// with the counts, more than those are one more copy.
+static int read_heavy(vg_circuit *c, EdgeSet &E, const unsigned long long *st)
+{
+    const long n_heavy = (long)st[3];
     E.heavy_host.assign(3 * (size_t)n_heavy, 0);
-    if (!n_heavy) return VG_OK;
+    if (n_heavy <= HEAVY_INLINE) {
+        if (n_heavy) memcpy(E.heavy_host.data(), st + 4, 3 * (size_t)n_heavy * 4);
+        return VG_OK;
+    }
     if (3 * n_heavy > E.cap_H) return vg_fail(VG_ERR_STATE, "heavy key list overflow");
     VG_CHECK_CUDA(cudaMemcpyAsync(E.heavy_host.data(), E.heavy, 3 * n_heavy * 4, cudaMemcpyDeviceToHost, c->ctx->stream));
     VG_CHECK_CUDA(cudaStreamSynchronize(c->ctx->stream));
     return VG_OK;
 }
 
-// Reads the edge counts of every layer (the caller synchronised the stream
-// after stats_host was copied) and rebuilds the sets whose edges did not fit.
-static int finish_edges(vg_circuit *c, const unsigned long long *stats_host)
+// Takes over the edge counts of every layer (read_edge_stats) after building
+// the layers again whose edges did not fit (summation gates), now that their
+// number is known.
+static int finish_edges(vg_circuit *c)
 {
-    bool refill = false;
-    for (int li = 1; li < c->depth; ++li)
-        for (int ph = 0; ph < 2; ++ph) {
-            EdgeSet &E = c->L[li].ph[ph];
-            const unsigned long long *st = stats_host + EDGE_STATS * (2 * li + ph);
-            if (!E.launched) continue;
-            if (st[0] >= (1ull << 31)) {   // too many edges: atomic path
-                E.launched = false;
-                continue;
+    for (bool again = true; again;) {
+        again = false;
+        for (int li = 1; li < c->depth; ++li) {
+            bool refill = false;
+            for (int ph = 0; ph < 2; ++ph) {
+                EdgeSet &E = c->L[li].ph[ph];
+                const unsigned long long *st = c->edge_stats_host.data() + EDGE_STATS * (2 * li + ph);
+                if (!E.launched) continue;
+                if (st[0] >= (1ull << 31)) E.launched = false;   // too many edges: atomic path
+                else if (st[2]) {
+                    VG_TRY(alloc_edges(c->ctx, E, (long)st[0]));
+                    refill = true;
+                }
             }
-            E.E = (long)st[0];
-            if (st[2]) {   // overflowed: exact size now known (rare: summation gates)
-                VG_TRY(alloc_edges(c->ctx, E, E.E));
-                refill = true;
-                E.ok = false;
-                continue;
-            }
-            E.n_medium = (long)st[1];
-            VG_TRY(read_heavy(c, E, (long)st[3]));
-            E.ok = true;
+            if (!refill) continue;
+            VG_CHECK_CUDA(cudaMemsetAsync(c->edge_stats + EDGE_STATS * 2 * li, 0, EDGE_STATS * 2 * 8, c->ctx->stream));
+            VG_TRY(launch_edges(c, li));
+            again = true;
         }
-    if (!refill) return VG_OK;
-    // the offsets are intact (the fill works on a copy): fill again with room
-    vg_ctx *ctx = c->ctx;
+        if (again) VG_TRY(read_edge_stats(c));
+    }
     for (int li = 1; li < c->depth; ++li)
         for (int ph = 0; ph < 2; ++ph) {
             EdgeSet &E = c->L[li].ph[ph];
-            if (!E.launched || E.ok || E.cap_E < E.E || E.E >= (1L << 31)) continue;
-            VG_TRY(fill_edges(c, li, ph));
-            unsigned long long st[EDGE_STATS];
-            VG_CHECK_CUDA(cudaMemcpyAsync(st, c->edge_stats + EDGE_STATS * (2 * li + ph), EDGE_STATS * 8,
-                                          cudaMemcpyDeviceToHost, ctx->stream));
-            VG_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
-            if (st[2]) continue;   // still does not fit: atomic path
+            const unsigned long long *st = c->edge_stats_host.data() + EDGE_STATS * (2 * li + ph);
+            if (!E.launched) continue;
+            E.E = (long)st[0];
             E.n_medium = (long)st[1];
-            VG_TRY(read_heavy(c, E, (long)st[3]));
+            VG_TRY(read_heavy(c, E, st));
             E.ok = true;
         }
     return VG_OK;
@@ -1763,12 +1889,10 @@ extern "C" int vg_circuit_upload(vg_ctx *ctx, int depth, const int *bit_length, 
         cudaError_t e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) return fail(vg_fail(VG_ERR_CUDA, "circuit upload: %s", cudaGetErrorString(e)));
     }
-    int rc = launch_all_edges(c);
-    if (rc == VG_OK) {
-        cudaError_t e = cudaStreamSynchronize(ctx->stream);
-        if (e != cudaSuccess) return fail(vg_fail(VG_ERR_CUDA, "circuit upload: %s", cudaGetErrorString(e)));
-        rc = finish_edges(c, c->edge_stats_host.data());
-    }
+    int rc = start_edges(c);
+    for (int i = 1; i < depth && rc == VG_OK; ++i) rc = launch_edges(c, i);
+    if (rc == VG_OK) rc = read_edge_stats(c);
+    if (rc == VG_OK) rc = finish_edges(c);
     if (rc != VG_OK) return fail(rc);
     *out = c;
     return VG_OK;
@@ -1895,6 +2019,10 @@ extern "C" int vg_circuit_build(vg_ctx *ctx, int d, const long *n, const uint8_t
     int rc = grow_dev(ctx, &c->staging, &c->staging_cap, stage_b);
     if (rc != VG_OK) return fail(rc);
     const unsigned grid_cap = 148u * 32u;
+    // a layer's edge sets follow its wires (as checked: invalid gates became
+    // dummies) and are built while the next layers are copied
+    rc = start_edges(c);
+    if (rc != VG_OK) return fail(rc);
     for (int fi = 0; fi < d; ++fi) {
         const long cnt = n[fi];
         const size_t wb = fi == 0 ? 8 : (size_t)index_bytes;   // the input layer's u are values (int64)
@@ -1913,6 +2041,7 @@ extern "C" int vg_circuit_build(vg_ctx *ctx, int d, const long *n, const uint8_t
             k_build_relay<<<std::min<unsigned>(grid_for(R.n, 256), grid_cap), 256, 0, ctx->stream>>>(
                 std::max(cnt, pad), R.n, R.ty, R.u, R.v);
             VG_LAUNCHED(ctx);
+            rc = launch_edges(c, 1);
         } else {
             const int li = fi + 1;
             DevLayer &D = c->L[li];
@@ -1925,21 +2054,20 @@ extern "C" int vg_circuit_build(vg_ctx *ctx, int d, const long *n, const uint8_t
                 k_build_layer<uint32_t><<<grid, 256, 0, ctx->stream>>>(sty, (const uint32_t *)su, (const uint32_t *)sv, cnt,
                                                                        D.n, prev, li, D.ty, D.u, D.v, c->err);
             VG_LAUNCHED(ctx);
+            rc = launch_edges(c, li);
         }
+        if (rc != VG_OK) return fail(rc);
     }
-    // edge sets from the checked wires (invalid gates became dummies), then one
-    // synchronisation for the error flag and the edge counts
-    rc = launch_all_edges(c);
-    if (rc != VG_OK) return fail(rc);
     unsigned long long e = 0;
     VG_CHECK_CUDA(cudaMemcpyAsync(&e, c->err, sizeof e, cudaMemcpyDeviceToHost, ctx->stream));
-    VG_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
+    rc = read_edge_stats(c);
+    if (rc != VG_OK) return fail(rc);
     if (e != ~0ull) {
         const int li = (int)(e >> 40);
         const long gi = (long)(e & ((1ull << 40) - 1));
         return fail(vg_fail(VG_ERR_ARG, "file layer %d gate %ld: invalid type or wire", li == 0 ? 0 : li - 1, gi));
     }
-    rc = finish_edges(c, c->edge_stats_host.data());
+    rc = finish_edges(c);
     if (rc != VG_OK) return fail(rc);
     if (bit_lengths)
         for (int i = 0; i < depth; ++i) bit_lengths[i] = bl[i];
