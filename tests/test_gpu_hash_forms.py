@@ -9,6 +9,7 @@ import pytest
 
 import _oracle as O
 import virgo_b200 as vb
+from virgo_b200 import transcript
 
 pytestmark = pytest.mark.gpu
 
@@ -61,3 +62,44 @@ def test_merkle_subtrees(kind, n):
         assert got.tobytes() == b"".join(tree)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("log_in", [10, 16, 17, 18])
+@pytest.mark.parametrize("gates", [2, 1 << 20])
+def test_proof_leaves_are_chains_of_all_slices(log_in, gates):
+    """A proof's committed leaves, whether their chains ran in one launch (the
+    circuits with 2^20 gates, up to 2^17 values) or went on after the mask
+    slice came (the others): on pairs, on threads and, for 2^18 values, on both."""
+    rng = np.random.default_rng(log_in)
+    n = 1 << log_in
+    layers = [(np.full(n, 3, np.uint8), rng.integers(0, 1 << 20, n), np.zeros(n, np.int64)),
+              (rng.integers(0, 2, gates).astype(np.uint8), rng.integers(0, n, gates), rng.integers(0, n, gates))]
+    s = vb.Session(layers)
+    try:
+        for seed in (3, 4):
+            recs = transcript.parse(s.prove(seed)[1])
+            roots = [d for t, d in recs if t == "C"][:2]
+            first = [d for t, d in recs if t == "I"]
+            assert len(first) >= 10 and len(first) % 2 == 0
+            for i, d in enumerate(first):   # l and h in turn
+                counts = int.from_bytes(d[8:16], "little")
+                nv, nd = counts >> 16, counts & 0xffff
+                assert nv == 65 and len(d) == 16 + 32 * (nv + nd)
+                values, nodes = d[16:16 + 32 * nv], d[16 + 32 * nv:]
+                h = bytes(32)
+                for k in range(nv):
+                    h = hashlib.sha3_256(values[32 * k:32 * k + 32] + h).digest()
+                assert h == nodes[-32:]
+                if i < 2:
+                    assert roots[i] in _folds(h, [nodes[32 * k:32 * k + 32] for k in range(nd - 1)])
+    finally:
+        s.close()
+
+
+def _folds(h, siblings):
+    """The roots that a leaf digest and its siblings can have, left and right
+    siblings together (the position is not in the record)."""
+    level = {h}
+    for x in siblings:
+        level = {hashlib.sha3_256(p).digest() for a in level for p in (a + x, x + a)}
+    return level

@@ -18,6 +18,14 @@ namespace {
 
 constexpr int HASH_THREADS = 128;
 
+__device__ __forceinline__ void load_digest(const uint64_t *p, uint64_t h[4])
+{
+    const ulonglong2 a = reinterpret_cast<const ulonglong2 *>(p)[0], b = reinterpret_cast<const ulonglong2 *>(p)[1];
+    h[0] = a.x;
+    h[1] = a.y;
+    h[2] = b.x;
+    h[3] = b.y;
+}
 __device__ __forceinline__ void load_digest2(const uint64_t *p, uint64_t w[8])
 {
     const ulonglong2 *q = (const ulonglong2 *)p;
@@ -89,6 +97,8 @@ __global__ void k_tree_leaves(const ulonglong2 *leaves, long n, long size, ulong
 // warp reads 32 consecutive k of one slice, 512 contiguous bytes per load; the
 // next slice's pair is loaded before the current hash), except the chains from
 // thread_chains on, which take a pair of lanes each (vg_leaf_chains chooses).
+// A launch may stop before the last slice and another go on from the digests
+// it left (jobs.first).
 __device__ __forceinline__ int chain_job(const ChainJobs &jobs, long t)
 {
     int q = 0;
@@ -103,8 +113,9 @@ __device__ __forceinline__ void thread_chain(const ChainJobs &jobs, long t)
     const fe *__restrict__ c = jobs.j[q].cw;
     const long n = jobs.j[q].n, half = n >> 1, k = t - jobs.j[q].begin;
     uint64_t h[4] = {0, 0, 0, 0};
-    fe a = c[k], b = c[k + half];
-    for (int s = 0; s < jobs.slices; ++s) {
+    if (jobs.first) load_digest(jobs.j[q].leaves + 4 * k, h);
+    fe a = c[(long)jobs.first * n + k], b = c[(long)jobs.first * n + k + half];
+    for (int s = jobs.first; s < jobs.slices; ++s) {
         fe na = a, nb = b;
         if (s + 1 < jobs.slices) {
             na = c[(long)(s + 1) * n + k];
@@ -129,8 +140,14 @@ __device__ __forceinline__ void pair_chain(const ChainJobs &jobs, long t, bool a
     uint32_t s25[25];
 #pragma unroll
     for (int i = 0; i < 4; ++i) s25[i] = 0;
-    fe a = c[k], b = c[k + half];
-    for (int s = 0; s < jobs.slices; ++s) {
+    if (jobs.first && active) {
+        uint64_t h[4];
+        load_digest(jobs.j[q].leaves + 4 * k, h);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s25[i] = vg::pair_half(h[i], odd);
+    }
+    fe a = c[(long)jobs.first * n + k], b = c[(long)jobs.first * n + k + half];
+    for (int s = jobs.first; s < jobs.slices; ++s) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) s25[4 + i] = s25[i];
         s25[0] = vg::pair_half(a.img, odd);
@@ -371,9 +388,9 @@ int vg_leaf_chains(vg_ctx *c, const ChainJobs &jobs_in)
     ChainJobs jobs = jobs_in;
     double bytes = 0;
     for (int q = 0; q < jobs.count; ++q)
-        bytes += 16.0 * jobs.slices * (double)jobs.j[q].n + 32.0 * (double)(jobs.j[q].n >> 1);
+        bytes += 16.0 * (jobs.slices - jobs.first) * (double)jobs.j[q].n + (jobs.first ? 64.0 : 32.0) * (double)(jobs.j[q].n >> 1);
     ProfScope ps(c, KF_LEAF_CHAIN, bytes);
-    if (use_warp_chains(c, jobs.total)) {
+    if (jobs.first == 0 && use_warp_chains(c, jobs.total)) {
         k_leaf_chains_warp<<<warp_chain_grid(jobs.total), WARP_CHAIN_THREADS, 0, c->stream>>>(jobs);
     } else {
         int T = (int)vg_tune_value(c->device, VG_TUNE_LEAF_THREADS);
@@ -387,21 +404,31 @@ int vg_leaf_chains(vg_ctx *c, const ChainJobs &jobs_in)
         else if (jobs.total < 24 * SCHEDULERS * 32) T = 64;
         const long rest = jobs.total - jobs.thread_chains;
         const unsigned grid = (unsigned)((jobs.thread_chains + T - 1) / T + (rest + T / 2 - 1) / (T / 2));
-#define VG_CHAINS_LAUNCH(TT)                                                                                    \
-    if (c->hash_kind == VG_HASH_SHA256)                                                                          \
-        k_leaf_chains<VG_HASH_SHA256, TT, 0><<<grid, TT, 0, c->stream>>>(jobs);                                 \
-    else if (rot == 1)                                                                                           \
-        k_leaf_chains<VG_HASH_SHA3_256, TT, 1><<<grid, TT, 0, c->stream>>>(jobs);                              \
-    else if (rot == 2)                                                                                           \
-        k_leaf_chains<VG_HASH_SHA3_256, TT, 2><<<grid, TT, 0, c->stream>>>(jobs);                              \
-    else if (rot == 3)                                                                                           \
-        k_leaf_chains<VG_HASH_SHA3_256, TT, 3><<<grid, TT, 0, c->stream>>>(jobs);                              \
-    else                                                                                                         \
-        k_leaf_chains<VG_HASH_SHA3_256, TT, 0><<<grid, TT, 0, c->stream>>>(jobs)
-        if (T == 64) VG_CHAINS_LAUNCH(64);
-        else if (T == 256) VG_CHAINS_LAUNCH(256);
-        else VG_CHAINS_LAUNCH(128);
+        // Room for no more CTAs on an SM than an even spread takes (by shared
+        // memory the kernel does not use): beside another stream's kernel the
+        // SMs come free one after another, and the first ones took up to 768
+        // threads each while others stayed without (73728 chains beside a
+        // sumcheck 1707 -> 1166 us; alone 1142).
+        const long even = (grid + 147) / 148;
+        const int smem = even > 1 && even < 768 / T ? (int)(((228L << 10) / even - 1024) & ~127L) : 0;
+#define VG_CHAINS_ONE(KIND, TT, ROT)                                                                                        \
+    {                                                                                                                       \
+        VG_CHECK_CUDA(cudaFuncSetAttribute(k_leaf_chains<KIND, TT, ROT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
+        k_leaf_chains<KIND, TT, ROT><<<grid, TT, smem, c->stream>>>(jobs);                                                  \
+    }
+#define VG_CHAINS_LAUNCH(TT)                                                      \
+    {                                                                             \
+        if (c->hash_kind == VG_HASH_SHA256) VG_CHAINS_ONE(VG_HASH_SHA256, TT, 0)  \
+        else if (rot == 1) VG_CHAINS_ONE(VG_HASH_SHA3_256, TT, 1)                 \
+        else if (rot == 2) VG_CHAINS_ONE(VG_HASH_SHA3_256, TT, 2)                 \
+        else if (rot == 3) VG_CHAINS_ONE(VG_HASH_SHA3_256, TT, 3)                 \
+        else VG_CHAINS_ONE(VG_HASH_SHA3_256, TT, 0)                               \
+    }
+        if (T == 64) VG_CHAINS_LAUNCH(64)
+        else if (T == 256) VG_CHAINS_LAUNCH(256)
+        else VG_CHAINS_LAUNCH(128)
 #undef VG_CHAINS_LAUNCH
+#undef VG_CHAINS_ONE
     }
     VG_LAUNCHED(c);
     return VG_OK;

@@ -86,6 +86,9 @@ void vg_pc_set_side(vg_pc *pc, vg_ctx *side);
 // all leaf chains and Merkle trees batched, the query answers for
 // (which, pos) as in vg_pc_query_batch, and the copies of every result into
 // pinned memory (out points there).
+// vg_pc_prove_begin enqueues what depends on priv alone; the
+// vg_pc_prove_deferred after it, with the same priv and `begun`, does the rest.
+int vg_pc_prove_begin(vg_pc *pc, const vg_fe *priv, int log_len);
 int vg_pc_prove_deferred(vg_pc *pc, const vg_fe *priv, int log_len, const vg_fe *pri_mask, long n_pri_mask,
                          const vg_fe *pub, const vg_fe *pub_mask, long n_pub_mask, const vg_fe *fri_r, int nlevels,
-                         int nq, const int *which, const long *pos, vg_pc_results *out);
+                         int nq, const int *which, const long *pos, bool begun, vg_pc_results *out);

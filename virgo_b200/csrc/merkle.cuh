@@ -24,6 +24,7 @@ struct ChainJob {
 struct ChainJobs {
     ChainJob j[MAX_HASH_JOBS];
     int count, slices;
+    int first;    // first slice: 0, or the leaves hold the digests of the slices before it and the chains go on from them
     long total;   // chains = sum of n / 2
     long thread_chains;   // of those, the first ones hashed by one thread each; the others by two lanes each
 };
