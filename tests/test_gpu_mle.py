@@ -2,6 +2,7 @@
 CTA, one chunk per CTA, chunks of several rows, looping CTAs), device and host
 inputs, against Python integers and the allocation-free entry point."""
 import ctypes
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import pytest
@@ -42,3 +43,36 @@ def test_mle_eval_sizes(log_n):
             assert (int(out[0][1]), int(out[0][0])) == mle(vals, r[:log_n])
     finally:
         ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("log_n", [3, 16, 18, 20])
+def test_contexts_that_follow_one_another_in_threads(log_n):
+    """Pinned blocks change hands between contexts of several threads: every
+    evaluation of a host table is its own table's."""
+    rng = np.random.default_rng(log_n)
+    r = rng.integers(0, P, (log_n, 2), dtype=np.int64)
+    tables = [rng.integers(0, P, (1 << log_n, 2), dtype=np.int64) for _ in range(4)]
+
+    def evaluate(ctx, vals):
+        out = np.zeros((1, 2), np.int64)
+        vb.check(vb.lib().vg_mle_eval(ctx.h, vals, 1 << log_n, r.ctypes.data_as(ctypes.c_void_p), log_n,
+                                      out.ctypes.data_as(ctypes.c_void_p)), "vg_mle_eval")
+        return out.tobytes()
+
+    def value(t):
+        ctx = vb.Context(0)
+        try:
+            return evaluate(ctx, t.ctypes.data_as(ctypes.c_void_p))
+        finally:
+            ctx.close()
+
+    ctx = vb.Context(0)
+    on_device = [ctx.buffer(t) for t in tables]
+    want = [evaluate(ctx, b.p) for b in on_device]
+    for b in on_device:
+        b.free()
+    ctx.close()
+    with ThreadPoolExecutor(4) as pool:
+        for _ in range(4):
+            assert list(pool.map(value, tables)) == want

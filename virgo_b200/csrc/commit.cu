@@ -238,7 +238,7 @@ static void pc_free(vg_pc *pc)
     pc->levels.clear();
     pc->nlevels = 0;
     pc->have_private = pc->have_public = false;
-    if (pc->hpin) cudaFreeHost(pc->hpin);
+    vg_pinned_give(pc->hpin);
     pc->hpin = nullptr;
     pc->hpin_cap = 0;
 }

@@ -135,6 +135,11 @@ void vg_release(vg_ctx *c, void *p);
 int vg_scratch(vg_ctx *ctx, size_t bytes, void **p);
 int vg_scratch2(vg_ctx *ctx, size_t bytes, void **p);
 int vg_partials(vg_ctx *ctx, size_t n, fe **p);
+// Pinned host blocks of at least `bytes` (cap receives the size), kept for the
+// next taker when given back; null is ignored.  Synchronise the streams that
+// use a block before giving it back.
+int vg_pinned_take(void **p, size_t bytes, size_t *cap);
+void vg_pinned_give(void *p);
 int vg_pinned(vg_ctx *ctx, size_t n, fe **p);
 // grid_sum's device words for the context's kernels (up to 14 values per sum)
 int vg_grid_scratch(vg_ctx *ctx, unsigned long long **gacc, unsigned **counter);

@@ -4,7 +4,9 @@
 // Context, device memory, error reporting, elementwise field ops and the
 // generic partial-sum reduction.
 #include "common.cuh"
+#include <map>
 #include <mutex>
+#include <unordered_map>
 
 static thread_local std::string g_err;
 
@@ -33,6 +35,87 @@ static void default_connections()
     std::call_once(once, [] { setenv("CUDA_DEVICE_MAX_CONNECTIONS", "32", 0); });
 }
 
+// Pinned host blocks.  Pinning costs 0.7 to 3.5 ms a block whatever its size,
+// and a new session needs seven (5 to 13 of the 8 to 16 ms of its first proof),
+// so blocks given back are kept for the next object: up to PINNED_HELD bytes in
+// all, and only while a context exists.  Blocks are given back after the
+// streams that use them were synchronised; pinned memory serves every device.
+struct PinnedBlocks {
+    std::mutex mu;
+    std::unordered_map<void *, size_t> size;   // blocks in use or kept, by address
+    std::multimap<size_t, void *> kept;
+    size_t held = 0;   // bytes kept
+    int contexts = 0;
+    void trim()        // with mu held
+    {
+        for (auto &b : kept) {
+            size.erase(b.second);
+            cudaFreeHost(b.second);
+        }
+        kept.clear();
+        held = 0;
+    }
+};
+constexpr size_t PINNED_MIN = 4u << 10, PINNED_LARGE = 16u << 20, PINNED_HELD = 128u << 20;
+static PinnedBlocks &pinned_blocks()
+{
+    static PinnedBlocks *b = new PinnedBlocks();   // outlives the CUDA runtime's own teardown
+    return *b;
+}
+
+int vg_pinned_take(void **p, size_t bytes, size_t *cap)
+{
+    // powers of two, so blocks of like sizes serve each other; large ones are not kept
+    size_t n = bytes;
+    if (bytes <= PINNED_LARGE)
+        for (n = PINNED_MIN; n < bytes;) n *= 2;
+    if (cap) *cap = n;
+    PinnedBlocks &B = pinned_blocks();
+    std::unique_lock<std::mutex> lock(B.mu);
+    auto it = B.kept.find(n);
+    if (it != B.kept.end()) {
+        *p = it->second;
+        B.held -= n;
+        B.kept.erase(it);
+        return VG_OK;
+    }
+    lock.unlock();   // others need not wait for the pinning
+    cudaError_t e = cudaMallocHost(p, n);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        lock.lock();
+        B.trim();
+        lock.unlock();
+        VG_CHECK_CUDA(cudaMallocHost(p, n));
+    }
+    lock.lock();
+    B.size[*p] = n;
+    return VG_OK;
+}
+
+void vg_pinned_give(void *p)
+{
+    if (!p) return;
+    PinnedBlocks &B = pinned_blocks();
+    std::lock_guard<std::mutex> lock(B.mu);
+    const size_t n = B.size[p];
+    if (B.contexts > 0 && n <= PINNED_LARGE && B.held + n <= PINNED_HELD) {
+        B.kept.emplace(n, p);
+        B.held += n;
+    } else {
+        B.size.erase(p);
+        cudaFreeHost(p);
+    }
+}
+
+static void count_context(int d)
+{
+    PinnedBlocks &B = pinned_blocks();
+    std::lock_guard<std::mutex> lock(B.mu);
+    B.contexts += d;
+    if (B.contexts == 0) B.trim();
+}
+
 extern "C" int vg_ctx_create(int device, vg_ctx **out)
 {
     if (!out) return vg_fail(VG_ERR_ARG, "vg_ctx_create: null out");
@@ -50,6 +133,7 @@ extern "C" int vg_ctx_create(int device, vg_ctx **out)
         delete c;
         return vg_fail(VG_ERR_CUDA, "cudaStreamCreate: %s", cudaGetErrorString(e));
     }
+    count_context(1);
     *out = c;
     return VG_OK;
 }
@@ -248,13 +332,14 @@ extern "C" int vg_ctx_destroy(vg_ctx *c)
     if (c->scratch2) cudaFree(c->scratch2);
     if (c->partials) cudaFree(c->partials);
     if (c->gsum) cudaFree(c->gsum);
-    if (c->pinned) cudaFreeHost(c->pinned);
-    for (void *q : c->retired_pinned) cudaFreeHost(q);
-    if (c->ring) cudaFreeHost(c->ring);
+    vg_pinned_give(c->pinned);
+    for (void *q : c->retired_pinned) vg_pinned_give(q);
+    vg_pinned_give(c->ring);
     for (cudaEvent_t ev : c->ring_ev)
         if (ev) cudaEventDestroy(ev);
     cudaStreamDestroy(c->stream);
     delete c;
+    count_context(-1);
     return VG_OK;
 }
 
@@ -351,7 +436,9 @@ int vg_h2d_staged(vg_ctx *c, void *dst, const void *src, size_t bytes)
     if (!c->ring) {
         for (auto &ev : c->ring_ev)
             if (!ev) VG_CHECK_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-        VG_CHECK_CUDA(cudaMallocHost((void **)&c->ring, vg_ctx::RING * RING_CHUNK));
+        void *ring;
+        VG_TRY(vg_pinned_take(&ring, vg_ctx::RING * RING_CHUNK, nullptr));
+        c->ring = (char *)ring;
     }
     for (size_t off = 0; off < bytes; off += RING_CHUNK) {
         const size_t len = std::min(RING_CHUNK, bytes - off);
@@ -402,7 +489,7 @@ int vg_pinned_grow(vg_ctx *c, void **p, size_t *cap, size_t bytes)
     if (bytes <= *cap) return VG_OK;
     size_t ncap = std::max(bytes, std::max(2 * *cap, (size_t)1 << 20));
     void *q = nullptr;
-    VG_CHECK_CUDA(cudaMallocHost(&q, ncap));
+    VG_TRY(vg_pinned_take(&q, ncap, &ncap));
     if (*p) c->retired_pinned.push_back(*p);
     *p = q;
     *cap = ncap;

@@ -446,8 +446,8 @@ extern "C" int vg_fft_gkr_destroy(vg_fft_gkr *f)
     vg_release(f->ctx, f->dev);
     for (cudaEvent_t e : f->ev)
         if (e) cudaEventDestroy(e);
-    if (f->host) cudaFreeHost(f->host);
-    if (f->parts_host) cudaFreeHost(f->parts_host);
+    vg_pinned_give(f->host);
+    vg_pinned_give(f->parts_host);
     delete f;
     return VG_OK;
 }

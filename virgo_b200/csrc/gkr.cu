@@ -2167,7 +2167,7 @@ extern "C" int vg_gkr_create(vg_ctx *ctx, const vg_circuit *c, vg_gkr **out)
     if (cudaMalloc(&g->round_counter, sizeof(unsigned)) != cudaSuccess) return fail("round counter");
     if (cudaMalloc(&g->vu, sizeof(fe)) != cudaSuccess) return fail("v_u");
     if (cudaMalloc(&g->rsync_dev, sizeof(fe)) != cudaSuccess) return fail("round challenge");
-    if (cudaMallocHost(&g->rsync_host, sizeof(fe)) != cudaSuccess) return fail("round challenge (pinned)");
+    if (vg_pinned_take((void **)&g->rsync_host, sizeof(fe), nullptr) != VG_OK) return fail("round challenge (pinned)");
     if (cudaMalloc(&g->heavy_parts, (size_t)MAX_HEAVY * HEAVY_PARTS * 4 * sizeof(fe)) != cudaSuccess)
         return fail("heavy partials");
     // on the context's stream: the streams are non-blocking, so a memset on
@@ -2209,12 +2209,12 @@ extern "C" int vg_gkr_destroy(vg_gkr *g)
     cudaFree(g->rg_acc);
     cudaFree(g->bgt);
     cudaFree(g->rec);
-    if (g->rec_host) cudaFreeHost(g->rec_host);
+    vg_pinned_give(g->rec_host);
     destroy_graphs(g);
     cudaFree(g->rdev);
-    if (g->rhost) cudaFreeHost(g->rhost);
+    vg_pinned_give(g->rhost);
     cudaFree(g->rsync_dev);
-    if (g->rsync_host) cudaFreeHost(g->rsync_host);
+    vg_pinned_give(g->rsync_host);
     delete g;
     return VG_OK;
 }
