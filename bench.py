@@ -62,10 +62,10 @@ COMMIT_BIN = os.path.join(ROOT, "oracle", "_ref", "commit_ref")
 FAMILIES = ["ntt_pass", "leaf_chain", "merkle_level", "fri_fold_leaf", "virtual_oracle", "eval_layer",
             "phase1_scatter", "phase2_scatter", "acc_finalize", "sumcheck_round", "reduce", "other", "gather_round"]
 # DRAM bytes / algorithmic bytes measured by ncu on a full-size launch of
-# the family's default kernel (profiles/k_round2_matmul256.txt: (403.0 +
-# 173.3) MB read + written for 604 MB algorithmic on a 2^23-entry paired
+# the family's default kernel (profiles/proof_kernels_matmul256.txt: (402.7 +
+# 80.4) MB read + written for 503 MB algorithmic on a 2^23-entry paired
 # round)
-TRAFFIC_RATIO = {"sumcheck_round": 0.954}
+TRAFFIC_RATIO = {"sumcheck_round": 0.960}
 HBM_BOUND = {"ntt_pass", "virtual_oracle", "eval_layer", "phase1_scatter", "phase2_scatter", "acc_finalize",
              "sumcheck_round", "reduce", "gather_round"}
 
@@ -76,7 +76,7 @@ HBM_BOUND = {"ntt_pass", "virtual_oracle", "eval_layer", "phase1_scatter", "phas
 # a property of the code and the circuit, not of the run.  The pipe's peak is
 # ncu's sm__inst_executed_pipe_alu.avg.peak_sustained, 2 warp instructions
 # per SM cycle, on 148 SMs at the run's median SM clock.
-ALU_WARP_INST_PER_PROOF = {"matmul256": 2.319e9}
+ALU_WARP_INST_PER_PROOF = {"matmul256": 1.856e9}
 # proofs the reference arm times per step (the step's sample)
 REF_SAMPLE_PER_STEP = 8
 ALU_PEAK_PER_SM_CYCLE = 2
@@ -887,7 +887,7 @@ def roofline(fam, hbm_peak, peak_kind, large=None):
             "traffic": round(per_launch * traffic) if traffic else None,
             "traffic_source": ("profile-derived constant, not measured in this run: the ratio of ncu "
                                "dram__bytes_read.sum + dram__bytes_write.sum to algorithmic bytes on a full-size "
-                               "launch (profiles/k_round2_matmul256.txt, %.3f), times this run's average "
+                               "launch (profiles/proof_kernels_matmul256.txt, %.3f), times this run's average "
                                "algorithmic bytes per launch" % traffic) if traffic else None,
             "peak_source": peak_kind, "launches_per_proof": f["launches"],
             "avg_launch_us": round(1000.0 * f["ms"] / f["launches"], 2), "bytes_per_launch": per_launch,
@@ -905,14 +905,14 @@ def roofline(fam, hbm_peak, peak_kind, large=None):
                          "the group start run inside its fused table build (k_gather_round2), so the family's "
                          "largest launches are there"}
                 if top == "sumcheck_round" and g["ms"] > 0 else None),
-            "alu_pipe_profile": {"frac_large_launches": 0.735, "frac_round_group": 0.33,
+            "alu_pipe_profile": {"frac_large_launches": 0.515, "frac_round_group": 0.228,
                                  "source": "profile-derived constants, not measured in this run: ncu "
                                            "sm__inst_executed_pipe_alu, pct of peak, of a paired round on a "
-                                           "2^23-entry table (profiles/k_round2_matmul256.txt) and a 64-CTA "
-                                           "round group (profiles/k_round_group_matmul256.txt)"},
+                                           "2^23-entry table and a 128-CTA round group "
+                                           "(profiles/proof_kernels_matmul256.txt)"},
             "note": "CUDA events on the launching stream; back-to-back launches share one event, so a "
                     "launch's time runs from the end of the one before it; the large launches are bound by "
-                    "the integer ALU pipe (ALU 73.5%, math-pipe throttle the top stall), the round groups of "
+                    "the multiply and ALU pipes (ALU 52%), the round groups of "
                     "the last 17 rounds of each phase by latency"}
 
 
