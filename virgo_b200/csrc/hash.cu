@@ -382,6 +382,30 @@ static long thread_chains(long chains)
     return full >= 6 || 2 * rest > SCHEDULERS ? chains : full * SCHEDULERS * 32;
 }
 
+// Shared memory of a chain launch that leaves room for `ctas` CTAs on an SM
+// (228 KB, of which a CTA takes 1 KB for itself), at most CHAIN_MAX_SMEM, the
+// one for two.
+static constexpr int spread_smem(long ctas) { return (int)(((228L << 10) / ctas - 1024) & ~127L); }
+constexpr int CHAIN_MAX_SMEM = spread_smem(2);
+
+// The kernel attribute belongs to the kernel on the device, not to a launch:
+// it is raised once to the largest launch's size, since setting it to the
+// launch's own size races with launches of other sizes from other threads (a
+// launch above the value of the moment is refused).
+template <int KIND, int T, int ROT>
+static int chain_smem_attribute(int dev)
+{
+    static std::mutex mu;
+    static std::vector<bool> done;
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev >= (int)done.size()) done.resize(dev + 1, false);
+    if (!done[dev]) {
+        VG_CHECK_CUDA(cudaFuncSetAttribute(k_leaf_chains<KIND, T, ROT>, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN_MAX_SMEM));
+        done[dev] = true;
+    }
+    return VG_OK;
+}
+
 int vg_leaf_chains(vg_ctx *c, const ChainJobs &jobs_in)
 {
     if (jobs_in.total < 1) return VG_OK;
@@ -410,11 +434,11 @@ int vg_leaf_chains(vg_ctx *c, const ChainJobs &jobs_in)
         // threads each while others stayed without (73728 chains beside a
         // sumcheck 1707 -> 1166 us; alone 1142).
         const long even = (grid + 147) / 148;
-        const int smem = even > 1 && even < 768 / T ? (int)(((228L << 10) / even - 1024) & ~127L) : 0;
-#define VG_CHAINS_ONE(KIND, TT, ROT)                                                                                        \
-    {                                                                                                                       \
-        VG_CHECK_CUDA(cudaFuncSetAttribute(k_leaf_chains<KIND, TT, ROT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
-        k_leaf_chains<KIND, TT, ROT><<<grid, TT, smem, c->stream>>>(jobs);                                                  \
+        const int smem = even > 1 && even < 768 / T ? spread_smem(even) : 0;
+#define VG_CHAINS_ONE(KIND, TT, ROT)                                          \
+    {                                                                         \
+        if (smem > 48 * 1024) VG_TRY((chain_smem_attribute<KIND, TT, ROT>(c->device))); \
+        k_leaf_chains<KIND, TT, ROT><<<grid, TT, smem, c->stream>>>(jobs);    \
     }
 #define VG_CHAINS_LAUNCH(TT)                                                      \
     {                                                                             \
