@@ -437,7 +437,8 @@ enum {
                                   memory (6 .. 10); a 2^n transform takes ceil(n / this) passes */
     VG_TUNE_NTT_TILE_LOG = 3,  /* NTT stage fusion width: log2 of the elements one CTA holds in a
                                   pass (10 .. 13; sub-DFTs of several columns share a CTA) */
-    VG_TUNE_LEAF_THREADS = 4,  /* threads per CTA of the per-thread leaf-chain kernels (64, 128, 256) */
+    VG_TUNE_LEAF_THREADS = 4,  /* threads per CTA of the leaf-chain kernels: 64 or 128 as they are;
+                                  256 (default) = chosen by the number of chains */
     VG_TUNE_LEAF_WARP_MAX = 5, /* Merkle leaf hashing: launches of at most this many SHA3 leaf
                                   chains hash each chain with a whole warp (25 lanes of the
                                   Keccak state, one per thread) instead of one thread per chain;

@@ -11,6 +11,7 @@
 static __constant__ uint32_t vg_pow2c[32];
 #include "hash.cuh"
 #include "merkle.cuh"
+#include "leaf_shape.h"
 
 void virgo_hash64_kind(int kind, const void *src, void *dst);   // host/src/hash_host.cpp
 
@@ -368,26 +369,6 @@ static int pow2_table(int dev)
     return VG_OK;
 }
 
-// How many of `chains` SHA3 chains get a thread each.  Every scheduler of the
-// chip (4 per SM) runs whole warps, and one warp of 32 chains keeps it busy for
-// a full chain's time, so a last round of warps on some of them costs as much
-// as one on all.  Up to half a warp per scheduler is left over as pairs of
-// lanes instead, whose warps take about half as long: 98304 chains (5.2 warps
-// per scheduler) 1.69 -> 1.57 ms, 24576 (1.3) 571 -> 436 us, 2048 569 -> 169
-// us.  From six warps on the rounds average out.
-constexpr long SCHEDULERS = 148 * 4;
-static long thread_chains(long chains)
-{
-    const long warps = (chains + 31) / 32, full = warps / SCHEDULERS, rest = warps % SCHEDULERS;
-    return full >= 6 || 2 * rest > SCHEDULERS ? chains : full * SCHEDULERS * 32;
-}
-
-// Shared memory of a chain launch that leaves room for `ctas` CTAs on an SM
-// (228 KB, of which a CTA takes 1 KB for itself), at most CHAIN_MAX_SMEM, the
-// one for two.
-static constexpr int spread_smem(long ctas) { return (int)(((228L << 10) / ctas - 1024) & ~127L); }
-constexpr int CHAIN_MAX_SMEM = spread_smem(2);
-
 // The kernel attribute belongs to the kernel on the device, not to a launch:
 // it is raised once to the largest launch's size, since setting it to the
 // launch's own size races with launches of other sizes from other threads (a
@@ -417,24 +398,12 @@ int vg_leaf_chains(vg_ctx *c, const ChainJobs &jobs_in)
     if (jobs.first == 0 && use_warp_chains(c, jobs.total)) {
         k_leaf_chains_warp<<<warp_chain_grid(jobs.total), WARP_CHAIN_THREADS, 0, c->stream>>>(jobs);
     } else {
-        int T = (int)vg_tune_value(c->device, VG_TUNE_LEAF_THREADS);
         const int rot = c->hash_kind == VG_HASH_SHA3_256 ? (int)vg_tune_value(c->device, VG_TUNE_LEAF_ROT) : 0;
         if (rot == 1 || rot == 2) VG_TRY(pow2_table(c->device));
-        jobs.thread_chains = rot == 3 ? thread_chains(jobs.total) : jobs.total;
-        // one warp more or less per scheduler matters while there are few: small
-        // CTAs spread them (131072 chains 2.26 ms in CTAs of 256, 1.99 of 64);
-        // CTAs of 128 put one warp of threads on every scheduler of an SM
-        if (jobs.thread_chains < jobs.total) T = 128;
-        else if (jobs.total < 24 * SCHEDULERS * 32) T = 64;
-        const long rest = jobs.total - jobs.thread_chains;
-        const unsigned grid = (unsigned)((jobs.thread_chains + T - 1) / T + (rest + T / 2 - 1) / (T / 2));
-        // Room for no more CTAs on an SM than an even spread takes (by shared
-        // memory the kernel does not use): beside another stream's kernel the
-        // SMs come free one after another, and the first ones took up to 768
-        // threads each while others stayed without (73728 chains beside a
-        // sumcheck 1707 -> 1166 us; alone 1142).
-        const long even = (grid + 147) / 148;
-        const int smem = even > 1 && even < 768 / T ? spread_smem(even) : 0;
+        const ChainShape shape = chain_shape(rot == 3, (int)vg_tune_value(c->device, VG_TUNE_LEAF_THREADS), jobs.total);
+        const int T = shape.threads, smem = shape.smem;
+        const unsigned grid = shape.grid;
+        jobs.thread_chains = shape.thread_chains;
 #define VG_CHAINS_ONE(KIND, TT, ROT)                                          \
     {                                                                         \
         if (smem > 48 * 1024) VG_TRY((chain_smem_attribute<KIND, TT, ROT>(c->device))); \

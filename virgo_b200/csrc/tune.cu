@@ -23,7 +23,7 @@ const Range RANGES[VG_TUNE_COUNT] = {
     {128, 512, 256, true},                  // ROUND_THREADS
     {6, 10, 10, false},                     // NTT_MAX_LOG
     {10, 13, 12, false},                    // NTT_TILE_LOG
-    {64, 256, 256, true},                   // LEAF_THREADS
+    {64, 256, 256, true},                   // LEAF_THREADS (256: by the number of chains, leaf_shape.h)
     {0, 1L << 24, 0, false},                // LEAF_WARP_MAX
     {1, 2, 2, false},                       // ROUND_FUSE
     {0, 3, 3, false},                       // LEAF_ROT
