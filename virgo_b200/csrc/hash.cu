@@ -400,7 +400,8 @@ int vg_leaf_chains(vg_ctx *c, const ChainJobs &jobs_in)
     } else {
         const int rot = c->hash_kind == VG_HASH_SHA3_256 ? (int)vg_tune_value(c->device, VG_TUNE_LEAF_ROT) : 0;
         if (rot == 1 || rot == 2) VG_TRY(pow2_table(c->device));
-        const ChainShape shape = chain_shape(rot == 3, (int)vg_tune_value(c->device, VG_TUNE_LEAF_THREADS), jobs.total);
+        const ChainForm form = c->hash_kind == VG_HASH_SHA256 ? CHAIN_SHA256 : (rot == 3 ? CHAIN_PAIRS : CHAIN_SHA3);
+        const ChainShape shape = chain_shape(form, (int)vg_tune_value(c->device, VG_TUNE_LEAF_THREADS), jobs.total);
         const int T = shape.threads, smem = shape.smem;
         const unsigned grid = shape.grid;
         jobs.thread_chains = shape.thread_chains;

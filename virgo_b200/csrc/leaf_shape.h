@@ -31,18 +31,29 @@ struct ChainShape {
     int smem;
 };
 
-// pairs: the kernel form that has pairs of lanes; knob: VG_TUNE_LEAF_THREADS
-inline ChainShape chain_shape(bool pairs, int knob, long chains)
+enum ChainForm { CHAIN_PAIRS, CHAIN_SHA3, CHAIN_SHA256 };   // SHA3 with pairs of lanes, SHA3 on threads, SHA-256
+
+// knob: VG_TUNE_LEAF_THREADS
+inline ChainShape chain_shape(ChainForm form, int knob, long chains)
 {
     ChainShape s;
-    s.thread_chains = pairs ? thread_chains(chains) : chains;
+    s.thread_chains = form == CHAIN_PAIRS ? thread_chains(chains) : chains;
     // one warp more or less per scheduler matters while there are few: small
     // CTAs spread them (131072 chains 2.26 ms in CTAs of 256, 1.99 of 64);
     // CTAs of 128 put one warp of threads on every scheduler of an SM.  64 and
     // 128 set by hand are taken as they are.
+    // SHA-256 takes CTAs of 256, two warps per scheduler that start together,
+    // where they come out even: 65 slices of 32768 chains (at most two warps
+    // per scheduler) 293 us against 334 in CTAs of 128 and 340 of 64, 65536
+    // (four) 579 against 619 and 632.  With an odd number they leave a warp's
+    // place empty and CTAs of 128 are faster: 4096 (one) 170 against 291,
+    // 49152 (three) 475 against 578, 131072 (seven) 1059 against 1148.
+    const long warps = (chains + 31) / 32, per_scheduler = (warps + SCHEDULERS - 1) / SCHEDULERS;
     if (knob != 256) s.threads = knob;
     else if (s.thread_chains < chains) s.threads = 128;
-    else s.threads = chains < 24 * SCHEDULERS * 32 ? 64 : 256;
+    else if (chains >= 24 * SCHEDULERS * 32) s.threads = 256;
+    else if (form == CHAIN_SHA256) s.threads = per_scheduler % 2 ? 128 : 256;
+    else s.threads = 64;
     const int T = s.threads;
     s.grid = (unsigned)((s.thread_chains + T - 1) / T + (chains - s.thread_chains + T / 2 - 1) / (T / 2));
     // Room for no more CTAs on an SM than an even spread takes (by shared
