@@ -145,6 +145,7 @@ int vg_pinned(vg_ctx *ctx, size_t n, fe **p);
 int vg_grid_scratch(vg_ctx *ctx, unsigned long long **gacc, unsigned **counter);
 int vg_twiddles(vg_ctx *ctx, fe root, int logn, const fe **lo, const fe **hi);
 bool vg_is_device_ptr(const void *p);
+bool vg_reads_in_place(const void *p, int device);   // reads_in_place (memory_place.h) of what p points to
 
 static inline unsigned grid_for(long n, int threads)
 {

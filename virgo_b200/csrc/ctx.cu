@@ -4,6 +4,7 @@
 // Context, device memory, error reporting, elementwise field ops and the
 // generic partial-sum reduction.
 #include "common.cuh"
+#include "memory_place.h"
 #include <map>
 #include <mutex>
 #include <unordered_map>
@@ -531,14 +532,29 @@ int vg_ctx_wait_for(vg_ctx *waiter, vg_ctx *signaler)
     return VG_OK;
 }
 
-bool vg_is_device_ptr(const void *p)
+static MemoryKind memory_kind(const void *p, int *owner)
 {
     cudaPointerAttributes a;
+    *owner = -1;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return MEMORY_HOST;
     }
-    return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
+    *owner = a.device;
+    return a.type == cudaMemoryTypeManaged ? MEMORY_MANAGED : a.type == cudaMemoryTypeDevice ? MEMORY_DEVICE : MEMORY_HOST;
+}
+
+bool vg_is_device_ptr(const void *p)
+{
+    int owner;
+    return memory_kind(p, &owner) != MEMORY_HOST;
+}
+
+bool vg_reads_in_place(const void *p, int device)
+{
+    int owner;
+    const MemoryKind kind = memory_kind(p, &owner);
+    return reads_in_place(p, kind, owner, device);
 }
 
 extern "C" int vg_dev_alloc(vg_ctx *c, size_t bytes, void **dev)

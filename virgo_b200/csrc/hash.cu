@@ -516,7 +516,7 @@ extern "C" int vg_merkle_tree(vg_ctx *c, const vg_digest *leaves, long n, vg_dig
     j.padded = n < sz;
     memcpy(j.pad, pad, sizeof j.pad);
     const vg_digest *src = leaves;
-    if (((uintptr_t)leaves & 15) || !vg_is_device_ptr(leaves)) {   // copied first; the kernel reads them in place
+    if (!vg_reads_in_place(leaves, c->device)) {   // copied first
         VG_CHECK_CUDA(cudaMemcpyAsync(tree + sz, leaves, n * sizeof(vg_digest), cudaMemcpyDeviceToDevice, c->stream));
         src = tree + sz;
     }
