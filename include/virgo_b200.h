@@ -479,8 +479,9 @@ int vg_tune_range(int key, long *lo, long *hi, long *def);
  * after one warm-up batch per candidate, the best of them counting; keeps a
  * candidate only if it beats the value in force by more than 3%, and leaves
  * the winners set for the sessions' device.  trials (optional, up to
- * max_trials) receives every timing.  Do not prove on the same device from
- * other threads meanwhile. */
+ * max_trials) receives every timing; the keys without effect are not timed,
+ * their values have the time of the settings in force.  Do not prove on the
+ * same device from other threads meanwhile. */
 typedef struct {
     int key;
     long value;

@@ -27,6 +27,7 @@ namespace {
 struct Knob {
     int key;
     std::vector<long> cands;
+    bool inert = false;   // accepted without effect: every value has the time of the settings in force
 };
 
 // candidates per parameter; the defaults are among them
@@ -37,8 +38,8 @@ const std::vector<Knob> &knobs()
         {VG_TUNE_ROUND_FUSE, {1, 2}},
         {VG_TUNE_ROUND_THREADS, {128, 256, 512}},
         {VG_TUNE_BETA_TABLE, {0, 1}},
-        {VG_TUNE_GROUP_SPLIT, {0, 1}},
-        {VG_TUNE_LAZY_FOLD, {0, 1}},
+        {VG_TUNE_GROUP_SPLIT, {0, 1}, true},
+        {VG_TUNE_LAZY_FOLD, {0, 1}, true},
         {VG_TUNE_GATHER_FUSE, {0, 1}},
         {VG_TUNE_NTT_MAX_LOG, {8, 9, 10}},
         {VG_TUNE_NTT_TILE_LOG, {11, 12, 13}},
@@ -95,9 +96,17 @@ extern "C" int vg_autotune(vg_session *const *ss, int n, unsigned seed, int reps
         return nt++;
     };
 
+    double in_force_ms = 0;   // of the settings in force, from the key before
     for (const Knob &kb : knobs()) {
         long cur = 0;
         if ((rc = vg_tune_get(dev, kb.key, &cur)) != VG_OK) return rc;
+        if (kb.inert) {
+            const int t = record(kb.key, cur, in_force_ms);
+            if (t < max_trials) trials[t].chosen = 1;
+            for (long v : kb.cands)
+                if (v != cur) record(kb.key, v, in_force_ms);
+            continue;
+        }
         double cur_ms = 0;
         if ((rc = time_batch(&cur_ms)) != VG_OK) return rc;
         int best_trial = record(kb.key, cur, cur_ms);
@@ -120,6 +129,7 @@ extern "C" int vg_autotune(vg_session *const *ss, int n, unsigned seed, int reps
             }
         }
         if ((rc = vg_tune_set(dev, kb.key, best)) != VG_OK) return rc;
+        in_force_ms = best_ms;
         if (best_trial < max_trials) trials[best_trial].chosen = 1;
     }
     if (n_trials) *n_trials = nt < max_trials ? nt : max_trials;
