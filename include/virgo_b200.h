@@ -383,7 +383,8 @@ int vg_session_prove_batch(vg_session *const *ss, int n, const unsigned *seeds, 
  *   vg_digest roots[2 + levels] (l, h, FRI level t); vg_fe all_sum[65];
  *   vg_fe inner; vg_fe fri_r[levels]; vg_fe final_cw[65 * n_final]
  *   (slice-major); int32 which[nq]; int64 pos[nq] (as for vg_pc_query_batch);
- *   vg_fe qvals[130 * nq]; vg_digest qpaths[32 * nq]. */
+ *   vg_fe qvals[130 * nq]; vg_digest qpaths[32 * nq].
+ * What a record or a path does not use of its place is zero. */
 int vg_session_write_proof(vg_session *s, const char *path);
 /* A session with a context and no circuit yet (vg_session_load gives it one). */
 int vg_session_new(vg_session **out);
