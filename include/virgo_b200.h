@@ -254,7 +254,7 @@ int vg_pc_query_step(vg_pc *pc, int lvl, long pow, vg_fe *values, vg_digest *pat
  * (0 = l, 1 = h, 2 + t = FRI level t) at position pos[q] (taken modulo half
  * the per-slice length) and returns 130 values (values[q*130 ..]) and its
  * authentication path (paths[q*32 ..], path_len[q] digests: siblings
- * bottom-up, then the leaf).  All arrays host. */
+ * bottom-up, then the leaf; the other rows zero).  All arrays host. */
 int vg_pc_query_batch(vg_pc *pc, int nq, const int *which, const long *pos, vg_fe *values, vg_digest *paths,
                       int *path_len);
 /* The whole commitment of one proof in one call and one synchronisation

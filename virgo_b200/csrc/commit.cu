@@ -140,7 +140,7 @@ __global__ void k_fri_fold(const fe *__restrict__ c, long n, int t, fe r, const 
 
 // Query answers for a batch: block q answers query q from codeword set
 // desc[which[q]] at position pos[q] (taken modulo n/2): 65 value pairs and the
-// authentication path (siblings bottom-up, then the leaf).
+// authentication path (siblings bottom-up, then the leaf; zeros up to 32 rows).
 struct QueryDesc {
     const fe *cw;
     const uint64_t *tree;
@@ -157,10 +157,10 @@ __global__ void k_gather_batch(const QueryDesc *__restrict__ desc, const int *__
         vals[(long)q * 130 + 2 * i] = d.cw[(long)i * d.n + p];
         vals[(long)q * 130 + 2 * i + 1] = d.cw[(long)i * d.n + p + h];
     }
-    if (i <= d.depth) {
+    if (i < 32) {   // depth < 28
         const long leaf = p + h;
         const long src = i < d.depth ? ((leaf >> i) ^ 1) : leaf;
-        for (int w = 0; w < 4; ++w) paths[((long)q * 32 + i) * 4 + w] = d.tree[4 * src + w];
+        for (int w = 0; w < 4; ++w) paths[((long)q * 32 + i) * 4 + w] = i <= d.depth ? d.tree[4 * src + w] : 0;
     }
 }
 

@@ -1081,9 +1081,9 @@ extern "C" int vg_session_write_proof(vg_session *s, const char *path)
     put(&nq, 4);
     put(&n_final, 8);
     put(&psize, 4);
-    // A record's folded pairs are set in a phase's last round only, a path to
-    // its own depth only; what the buffers hold beside those (earlier proofs'
-    // values, or another object's) does not go into the file.
+    // A record's folded pairs are set in a phase's last round only; what the
+    // buffer holds beside those (earlier proofs' values, or another object's)
+    // does not go into the file.
     std::vector<F> rec((size_t)nrec * 9, F(0));
     auto copy_rec = [&](int i, int n) {
         if (i < nrec) std::copy(r.rec + 9 * (size_t)i, r.rec + 9 * (size_t)i + n, rec.begin() + 9 * (size_t)i);
@@ -1107,13 +1107,7 @@ extern "C" int vg_session_write_proof(vg_session *s, const char *path)
         put(&p, 8);
     }
     put(r.pc.qvals, (size_t)nq * 130 * sizeof(vg_fe));
-    const int L = C.circuit[0].bit_length;
-    std::vector<vg_digest> paths((size_t)nq * 32, vg_digest{});
-    for (int q = 0; q < nq; ++q) {
-        const int n = (r.which[q] < 2 ? L - 2 : L - (r.which[q] - 2) - 3) + 1;
-        std::copy(r.pc.qpaths + 32 * (size_t)q, r.pc.qpaths + 32 * (size_t)q + n, paths.begin() + 32 * (size_t)q);
-    }
-    put(paths.data(), paths.size() * sizeof(vg_digest));
+    put(r.pc.qpaths, (size_t)nq * 32 * sizeof(vg_digest));
     if (fclose(f) != 0) ok = false;
     if (!ok) return vg_fail(VG_ERR_ARG, "vg_session_write_proof: writing %s failed", path);
     return VG_OK;
