@@ -197,15 +197,6 @@ __device__ __forceinline__ void block_sum(fe (&v)[K], fe *sm)
 // additions over shuffles (block_sum) is five dependent steps of some 60
 // clocks each at two levels, then again over the CTAs' partials.
 constexpr int LIMBS = 6;   // limbs of a field element
-__device__ __forceinline__ fe fe_from_limbs(unsigned long long i0, unsigned long long i1, unsigned long long i2,
-                                            unsigned long long r0, unsigned long long r1, unsigned long long r2)
-{
-    // limb sums below 2^40: s0 + 2^21 s1 + 2^42 s2 mod p, each term below 2^62
-    fe x;
-    x.img = vg::canon64(i0 + (i1 << 21) + ((i2 << 42) & vg::P) + (i2 >> 19));
-    x.real = vg::canon64(r0 + (r1 << 21) + ((r2 << 42) & vg::P) + (r2 >> 19));
-    return x;
-}
 // limb sums of x over the calling warp (all 32 lanes), the same in every lane
 __device__ __forceinline__ void warp_limbs(fe x, uint32_t (&l)[LIMBS])
 {
@@ -259,7 +250,7 @@ __device__ __forceinline__ bool grid_sum(const fe (&acc)[K], uint32_t (&sw)[16][
     __shared__ unsigned long long sl[LIMBS * K];
     if (t < LIMBS * K) sl[t] = s;
     __syncthreads();
-    if (t < K) tot[t] = fe_from_limbs(sl[6 * t], sl[6 * t + 1], sl[6 * t + 2], sl[6 * t + 3], sl[6 * t + 4], sl[6 * t + 5]);
+    if (t < K) tot[t] = vg::fe_from_limbs(sl[6 * t], sl[6 * t + 1], sl[6 * t + 2], sl[6 * t + 3], sl[6 * t + 4], sl[6 * t + 5]);
     __syncthreads();
     return true;
 }

@@ -46,11 +46,10 @@ VG_HD uint64_t subp(uint64_t a, uint64_t b)
 }
 VG_HD uint64_t negp(uint64_t a) { return a ? P - a : 0; }
 
-// 64 x 64 -> 128 bits.  On the device the 128-bit type compiles to four
-// 32 x 32 wide multiplies and three carries; a low and a high product formed
-// separately (a * b, __umul64hi) take seven multiplies, and the multiply pipe
-// (one wide multiply per SM and clock) bounds every field kernel: an F_p2
-// product took 30.1 clocks per warp that way, 26.8 through this type.
+// 64 x 64 -> 128 bits, as one 128-bit product rather than a low and a high one
+// formed separately (a * b, __umul64hi): the multiply pipe bounds the field
+// kernels, and an F_p2 product took 30.1 clocks per warp that way, 26.8 through
+// this type (measured; the halves share their partial products).
 typedef unsigned __int128 u128;
 VG_HD u128 mul128(uint64_t a, uint64_t b) { return (u128)a * b; }
 
@@ -59,7 +58,10 @@ VG_HD uint64_t foldp(uint64_t x) { return (x & P) + (x >> 61); }
 // x mod p, canonical, for x < 2p: x + 1 reaches 2^61 exactly when x >= p.
 VG_HD uint64_t canonp(uint64_t x) { return (x + ((x + 1) >> 61)) & P; }
 
-// x mod p as (x & p) + (x >> 61), for x < 2^125: below 2^64.
+// x mod p as (x & p) + (x >> 61), for x <= 7 * 2^122: x >> 61 is at most
+// 7 * 2^61 and x & p at most p, so the sum stays below 2^64.  The callers' sums
+// are at most 6 p^2, which folds to at most 7p; with a canonical addend that is
+// 8p - 1 = 2^64 - 9, the top of canon64's range.
 VG_HD uint64_t fold128(u128 x)
 {
     const uint64_t lo = (uint64_t)x, hi = (uint64_t)(x >> 64);
@@ -159,6 +161,16 @@ VG_HD fe fe_fold(fe x0, fe x1, fold_r f)
 }
 
 VG_HD fe fe_double(fe a) { return a + a; }
+
+// The element whose components are given as sums of 21-, 21- and 19-bit limbs
+// (i0 + 2^21 i1 + 2^42 i2, and r likewise) over at most 2^21 values, so each sum
+// is below 2^42: i1 << 21 is below 2^63, the 2^42 term splits into at most p and
+// i2 >> 19 below 2^21, i0 is below 2^42, and the four stay below 2^64 - 9.
+VG_HD fe fe_from_limbs(uint64_t i0, uint64_t i1, uint64_t i2, uint64_t r0, uint64_t r1, uint64_t r2)
+{
+    return fe_make(canon64(r0 + (r1 << 21) + ((r2 << 42) & P) + (r2 >> 19)),
+                   canon64(i0 + (i1 << 21) + ((i2 << 42) & P) + (i2 >> 19)));
+}
 
 // Operands in F_p (imaginary part zero), such as every layer value of a
 // circuit (integer inputs, gates with coefficients in F_p): two products of

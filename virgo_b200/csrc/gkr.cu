@@ -1103,7 +1103,7 @@ __global__ void __launch_bounds__(RG_THREADS) k_round_group(const fe *__restrict
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const unsigned long long *p = lim + t * RG_LIMBS + k * LIMBS;
-            x[k] = fe_from_limbs(p[0], p[1], p[2], p[3], p[4], p[5]);
+            x[k] = vg::fe_from_limbs(p[0], p[1], p[2], p[3], p[4], p[5]);
         }
         rg_sums_end(x);
         fe *o = rec + 9 * (G.slot0 + t);
