@@ -659,9 +659,12 @@ static int ensure_pinned(vg_pc *pc, size_t elems)
 // The second stream of a whole commitment.  Everything about the mask slices
 // (single transforms, all latency, some 100 us in a row) runs there beside the
 // data slices.  From BESIDE_MIN on the hash chains of l, a third of the hashing,
-// run there too while the first stream takes in and encodes the public half
-// (2^20 values from host memory 20.1 -> 18.7 ms); for small commitments they
-// only slow the short kernels of the first stream down (2^15 903 -> 1120 us).
+// run there too while the first stream takes in and encodes the public half.
+// From there on it was never slower: 2^20 and 2^22 values from host memory 19.3
+// -> 18.4 and 85.1 -> 79.0 ms with SHA3, 13.2 -> 12.2 and 62.0 -> 55.8 with
+// SHA-256, values on the device the same within 1%.  Below, host arrays gain 1
+// to 6% from 2^15 values on, but device arrays with SHA-256 lose: 2^14 values 526
+// -> 579 us, 2^17 1.76 -> 1.89 ms, 2^19 5.81 -> 5.91 ms.
 // Every buffer belongs to the first stream: the second one starts after what
 // is queued there (fork) and the first continues after it (join) before
 // anything is reused or freed; an error in between waits for the second stream

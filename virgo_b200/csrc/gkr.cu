@@ -884,7 +884,7 @@ struct RoundGroup {
 // the value at 1 minus the other two.  acc[0] and acc[2] collect the x^2 terms
 // and the values at 0; with FULL acc[1] collects the values at 1 (three
 // products; rg_sums_end turns it into the x term), without it the x term is
-// left out (the group's epilogue forms it from the round's claim): two
+// left out (rg_derive forms it from the round's claim): two
 // products, each added inside its last fold.
 template <bool FULL = true>
 __device__ __forceinline__ void rg_sums(fe v0, fe v1, fe a0, fe a1, fe m0, fe m1, fe (&acc)[3])

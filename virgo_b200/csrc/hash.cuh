@@ -245,6 +245,8 @@ __device__ __forceinline__ void keccak_f_warp(uint32_t &lo, uint32_t &hi, const 
 }
 
 // ---- Keccak-f[1600] on a pair of lanes ----
+// Bit interleaving, the Keccak team's published way of running the 64-bit words
+// on 32-bit registers (Keccak implementation overview), over two lanes.
 // Lanes 2j and 2j + 1 of a warp share a permutation: the even one holds the
 // even-numbered bits of the 25 words, the odd one the odd-numbered bits, 32
 // each.  Bitwise steps and rotations by an even amount stay inside a lane (one

@@ -577,11 +577,12 @@ public:
 // Whether the commitment's first part is enqueued before the sumcheck rather
 // than with the rest after it: for circuits of up to six gates (the input's
 // relay layer among them) per input value.  Their proofs wait for the
-// commitment at the end (16x16 matmul, 1.1 gates per value: 3.60 -> 3.37 ms;
-// 64x64 matmul, 5: 3.75 -> 3.56; SHA-256 of 4 blocks, 4.8: 4.06 -> 3.94, six in
-// flight 16.7 -> 16.2).  Larger ones wait for the sumcheck, which the hashing
-// then only holds up sooner (random circuit, 9: 4.40 -> 4.44, eight in flight
-// 22.6 -> 23.3; 256x256 matmul, 257: 6.80 -> 6.82, eight in flight 44.9 -> 46.3).
+// commitment at the end; larger ones wait for the sumcheck, which the hashing
+// then only holds up sooner.  Proofs of 2^17 values, one at a time: 1 gate per
+// value 3.46 -> 3.33 ms, 3 3.51 -> 3.39, 6 3.66 -> 3.56, 7 3.72 -> 3.69, 8 3.78
+// -> 3.81, 9 3.84 -> 3.93, 12 4.22 -> 4.28; six in flight 15.9 -> 15.7 ms at 1,
+// 1 to 2% slower from 6 on.  2^18 and 2^20 values: within 2% either way, gains
+// up to 3 and 6 gates, losses from 7 on.
 static bool commit_first(const layered_circuit &C)
 {
     const int L = C.circuit[0].bit_length;
