@@ -430,9 +430,10 @@ void vg_free(void *p);
  * 256x256 matmul proof. */
 enum {
     VG_TUNE_GROUP_START = 0,   /* sumcheck tile: table length (power of two, 2^11 .. 2^22) at
-                                  which a phase's remaining rounds run as round groups (chunks of
-                                  2048 entries folded up to 10 rounds in shared memory, one CTA
-                                  per chunk) instead of one launch per round */
+                                  which a phase's remaining rounds, up to 20, run as one round
+                                  group (CTAs fold chunks of 64 to 1024 entries in shared memory,
+                                  the last one folds on what they leave) instead of one launch
+                                  per round */
     VG_TUNE_ROUND_THREADS = 1, /* threads per CTA of the one-round kernel (128, 256, 512) */
     VG_TUNE_NTT_MAX_LOG = 2,   /* NTT radix: log2 of the largest sub-DFT one pass runs in shared
                                   memory (6 .. 10); a 2^n transform takes ceil(n / this) passes */
