@@ -141,6 +141,7 @@ int vg_partials(vg_ctx *ctx, size_t n, fe **p);
 int vg_pinned_take(void **p, size_t bytes, size_t *cap);
 void vg_pinned_give(void *p);
 int vg_pinned(vg_ctx *ctx, size_t n, fe **p);
+void vg_gkr_context_gone(const vg_ctx *x);   // gkr.cu: x is about to be destroyed, its stream is done
 // grid_sum's device words for the context's kernels (up to 14 values per sum)
 int vg_grid_scratch(vg_ctx *ctx, unsigned long long **gacc, unsigned **counter);
 int vg_twiddles(vg_ctx *ctx, fe root, int logn, const fe **lo, const fe **hi);

@@ -319,6 +319,7 @@ extern "C" int vg_ctx_destroy(vg_ctx *c)
     if (!c) return VG_OK;
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
+    vg_gkr_context_gone(c);
     for (auto &p : c->prof) {
         cudaEventDestroy(p.a);
         cudaEventDestroy(p.b);

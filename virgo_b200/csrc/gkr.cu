@@ -1560,6 +1560,22 @@ struct vg_circuit {
     std::vector<unsigned long long> edge_stats_host;
 };
 
+// Which objects may have work on which circuit in their streams.  A circuit's
+// memory is given back once those streams are done; no stream of another
+// circuit is waited for.  (A wait for the whole device is an error while any
+// stream of it is being captured, and costs that capture: a session that closed
+// made other sessions' proofs fail.)  An object leaves when it is destroyed or
+// its context is, its stream done either way.
+struct Uses {
+    std::mutex mu;
+    std::vector<std::pair<vg_gkr *, const vg_circuit *>> list;
+};
+static Uses &uses()
+{
+    static Uses *u = new Uses();   // outlives objects that are destroyed at exit
+    return *u;
+}
+
 // One deferred round launch (k_round, k_round2 or k_round_group), held until
 // the next flush so that a phase's rounds are issued together: after one H2D
 // copy of their challenges, plainly or as a captured CUDA graph.
@@ -1854,7 +1870,11 @@ extern "C" int vg_circuit_upload(vg_ctx *ctx, int depth, const int *bit_length, 
     c->device = ctx->device;
     c->depth = depth;
     c->L.resize(depth);
-    auto fail = [&](int rc) { vg_circuit_destroy(c); return rc; };
+    auto fail = [&](int rc) {
+        cudaStreamSynchronize(ctx->stream);   // what was enqueued before the error
+        vg_circuit_destroy(c);
+        return rc;
+    };
     for (int i = 0; i < depth; ++i) {
         DevLayer &D = c->L[i];
         D.bl = bit_length[i];
@@ -1898,6 +1918,8 @@ extern "C" int vg_circuit_upload(vg_ctx *ctx, int depth, const int *bit_length, 
     return VG_OK;
 }
 
+static void wait_for_users(const vg_circuit *c);
+
 extern "C" int vg_circuit_destroy(vg_circuit *c)
 {
     if (!c) return VG_OK;
@@ -1906,7 +1928,7 @@ extern "C" int vg_circuit_destroy(vg_circuit *c)
     int cur = 0;
     cudaGetDevice(&cur);
     cudaSetDevice(c->device);
-    cudaDeviceSynchronize();
+    wait_for_users(c);
     for (auto &D : c->L) {
         cudaFree(D.ty);
         cudaFree(D.u);
@@ -1978,7 +2000,10 @@ extern "C" int vg_circuit_build(vg_ctx *ctx, int d, const long *n, const uint8_t
         c->cap.resize(depth, 0);
     }
     auto fail = [&](int rc) {
-        if (!*inout) vg_circuit_destroy(c);
+        if (!*inout) {
+            cudaStreamSynchronize(ctx->stream);   // what was enqueued before the error
+            vg_circuit_destroy(c);
+        }
         return rc;
     };
     if (!c->err && cudaMalloc(&c->err, sizeof(unsigned long long)) != cudaSuccess) {
@@ -2083,6 +2108,40 @@ extern "C" int vg_circuit_depth(const vg_circuit *c, int *depth)
 }
 
 // ---------------------------------------------------------------------- GKR
+template <typename Gone>
+static void drop_uses(Uses &U, Gone gone)
+{
+    U.list.erase(std::remove_if(U.list.begin(), U.list.end(), gone), U.list.end());
+}
+static void add_use(vg_gkr *g, const vg_circuit *c)
+{
+    Uses &U = uses();
+    std::lock_guard<std::mutex> lock(U.mu);
+    const std::pair<vg_gkr *, const vg_circuit *> use(g, c);
+    if (std::find(U.list.begin(), U.list.end(), use) == U.list.end()) U.list.push_back(use);
+}
+static void wait_for_users(const vg_circuit *c)
+{
+    Uses &U = uses();
+    std::lock_guard<std::mutex> lock(U.mu);
+    for (const auto &use : U.list)
+        if (use.second == c) cudaStreamSynchronize(use.first->ctx->stream);
+    drop_uses(U, [&](const auto &use) { return use.second == c; });
+}
+// the stream of g, or of every object of context x, is done
+static void drop_uses_of(const vg_gkr *g)
+{
+    Uses &U = uses();
+    std::lock_guard<std::mutex> lock(U.mu);
+    drop_uses(U, [&](const auto &use) { return use.first == g; });
+}
+void vg_gkr_context_gone(const vg_ctx *x)
+{
+    Uses &U = uses();
+    std::lock_guard<std::mutex> lock(U.mu);
+    drop_uses(U, [&](const auto &use) { return use.first->ctx == x; });
+}
+
 // Points g at circuit c, reusing every buffer that is large enough (a server
 // proving circuits of changing shapes then allocates only when one grows,
 // and cudaFree's device-wide synchronisation stays out of the proofs).
@@ -2092,6 +2151,7 @@ static int gkr_bind(vg_gkr *g, const vg_circuit *c)
         cudaGetLastError();
         return vg_fail(VG_ERR_OOM, "vg_gkr: %s allocation failed", what);
     };
+    add_use(g, c);
     long total = 0;
     // each layer on a 256-byte boundary (the paired rounds load 32 bytes at a time)
     for (int i = 1; i < c->depth; ++i) total += (c->L[i].n + 15) / 16 * 16;
@@ -2196,6 +2256,7 @@ extern "C" int vg_gkr_destroy(vg_gkr *g)
 {
     if (!g) return VG_OK;
     cudaStreamSynchronize(g->ctx->stream);
+    drop_uses_of(g);
     cudaFree(g->vals_slab);
     for (int b = 0; b < 2; ++b)
         for (int k = 0; k < 3; ++k) cudaFree(g->buf[b][k]);

@@ -292,10 +292,10 @@ extern "C" int vg_server_destroy(vg_server *s)
     }
     s->cv_work.notify_all();
     for (auto &t : s->workers) t.join();
-    // give the pool's unused reserve back to the device
+    // give the pool's unused reserve back to the device (the workers' sessions
+    // waited for their streams when they were destroyed)
     cudaMemPool_t pool;
     cudaSetDevice(s->device);
-    cudaDeviceSynchronize();
     if (cudaDeviceGetDefaultMemPool(&pool, s->device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
     cudaGetLastError();
     delete s;
