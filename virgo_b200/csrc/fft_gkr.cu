@@ -360,7 +360,7 @@ struct vg_fft_gkr {
     const void *g_key[3] = {nullptr, nullptr, nullptr};   // dev, host, parts_host at capture
     long long g_launched = 0;   // kernels in the graph
     bool g_seen = false;        // the last plain run had the current key
-    bool g_off = false;         // a capture failed: plain launches from then on
+    int g_failed = 0;           // captures lost; plain launches from MAX_LOST_CAPTURES on
 };
 
 // VIRGO_GRAPHS=0 turns the side proof's graph off (plain launches)
@@ -452,14 +452,13 @@ extern "C" int vg_fft_gkr_destroy(vg_fft_gkr *f)
     return VG_OK;
 }
 
-int vg_fft_gkr_launch(vg_fft_gkr *f, int lg, unsigned seed)
+// One run enqueued; *capturing (null: no capture) is set while it is being
+// captured, so still set when the capture was lost, in which case nothing ran.
+static int fg_enqueue(vg_fft_gkr *f, int lg, unsigned seed, bool *capturing)
 {
-    if (!f) return vg_fail(VG_ERR_ARG, "vg_fft_gkr_launch: null argument");
-    if (lg < 1 || lg > f->max_lg) return vg_fail(VG_ERR_ARG, "vg_fft_gkr: lg %d outside 1..%d", lg, f->max_lg);
-    if (f->pending) return vg_fail(VG_ERR_STATE, "vg_fft_gkr_launch: the previous run was not finished");
     vg_ctx *c = f->ctx;
     f->t0 = std::chrono::steady_clock::now();
-    const bool graphs = fg_graphs_enabled() && !f->g_off && !c->profiling;
+    const bool graphs = fg_graphs_enabled() && f->g_failed < MAX_LOST_CAPTURES && !c->profiling;
     if (graphs && f->gexec && f->g_lg == lg && f->g_seed == seed && f->g_key[0] == f->dev && f->g_key[1] == f->host &&
         f->g_key[2] == f->parts_host) {
         // H, prod_blocks and the host record pointer are those of the captured run
@@ -584,10 +583,11 @@ int vg_fft_gkr_launch(vg_fft_gkr *f, int lg, unsigned seed)
     // capture when the previous plain run had the same size, seed and buffers
     const bool same_key = f->g_lg == lg && f->g_seed == seed && f->g_key[0] == f->dev && f->g_key[1] == f->host &&
                           f->g_key[2] == f->parts_host;
-    const bool capture = graphs && f->g_seen && same_key;
+    const bool capture = capturing && graphs && f->g_seen && same_key;
     CaptureGuard guard;
     if (capture) {
         fg_drop_graph(f);
+        *capturing = true;
         VG_CHECK_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
         guard.s = c->stream;
         guard.active = true;
@@ -680,13 +680,10 @@ int vg_fft_gkr_launch(vg_fft_gkr *f, int lg, unsigned seed)
         if (e == cudaSuccess) e = cudaGraphInstantiate(&f->gexec, graph, 0);
         if (graph) cudaGraphDestroy(graph);
         if (e != cudaSuccess) {
-            // nothing of this run executed: launch it plainly, and from now on
-            cudaGetLastError();
             f->gexec = nullptr;
-            f->g_off = true;
-            c->launches = launches0;
-            return vg_fft_gkr_launch(f, lg, seed);
+            return vg_fail(VG_ERR_CUDA, "fft_gkr capture: %s", cudaGetErrorString(e));
         }
+        *capturing = false;
         f->g_launched = c->launches - launches0;
         VG_CHECK_CUDA(cudaGraphLaunch(f->gexec, c->stream));
     } else if (graphs) {
@@ -703,6 +700,24 @@ int vg_fft_gkr_launch(vg_fft_gkr *f, int lg, unsigned seed)
     f->lg = lg;
     f->pending = true;
     return VG_OK;
+}
+
+int vg_fft_gkr_launch(vg_fft_gkr *f, int lg, unsigned seed)
+{
+    if (!f) return vg_fail(VG_ERR_ARG, "vg_fft_gkr_launch: null argument");
+    if (lg < 1 || lg > f->max_lg) return vg_fail(VG_ERR_ARG, "vg_fft_gkr: lg %d outside 1..%d", lg, f->max_lg);
+    if (f->pending) return vg_fail(VG_ERR_STATE, "vg_fft_gkr_launch: the previous run was not finished");
+    const long long launches0 = f->ctx->launches;
+    bool capturing = false;
+    const int rc = fg_enqueue(f, lg, seed, &capturing);
+    if (rc == VG_OK || !capturing) return rc;
+    // the capture was lost (another thread of the program waited for the
+    // device, say) and nothing of this run executed: launched plainly
+    cudaGetLastError();
+    ++f->g_failed;
+    f->ctx->launches = launches0;
+    vg_gkr_tables_discard(f->tables);
+    return fg_enqueue(f, lg, seed, nullptr);
 }
 
 int vg_fft_gkr_finish(vg_fft_gkr *f, vg_fft_gkr_stats *st, vg_fe *msgs, vg_fe *vals)

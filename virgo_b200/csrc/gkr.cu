@@ -1673,7 +1673,7 @@ struct vg_gkr {
     // time it comes, replayed from then on)
     std::vector<PhaseGraph> graphs;
     std::vector<uint64_t> seen;
-    bool graphs_off = false;
+    int graphs_failed = 0;               // captures lost; plain launches from MAX_LOST_CAPTURES on
     long long graph_replays = 0, graph_captures = 0;
 };
 
@@ -2841,7 +2841,8 @@ static int exec_pending(vg_gkr *g)
     };
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     VG_CHECK_CUDA(cudaStreamIsCapturing(c->stream, &cs));
-    if (!rg_graphs_enabled() || g->graphs_off || c->profiling || cs != cudaStreamCaptureStatusNone) return issue();
+    if (!rg_graphs_enabled() || g->graphs_failed >= MAX_LOST_CAPTURES || c->profiling || cs != cudaStreamCaptureStatusNone)
+        return issue();
 
     std::vector<uint64_t> key;
     key.reserve(4 + 24 * launches.size());
@@ -2896,18 +2897,22 @@ static int exec_pending(vg_gkr *g)
     // second sight: capture, instantiate, launch
     if (g->graphs.size() >= 256) destroy_graphs(g);
     const long launches0 = c->launches;
-    VG_CHECK_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
-    const int rc = issue();
+    cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed);
+    int rc = VG_OK;
     cudaGraph_t graph = nullptr;
-    cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
+    if (e == cudaSuccess) {
+        rc = issue();
+        e = cudaStreamEndCapture(c->stream, &graph);
+    }
     cudaGraphExec_t exec = nullptr;
     if (rc == VG_OK && e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
     if (graph) cudaGraphDestroy(graph);
     if (rc != VG_OK || e != cudaSuccess) {
-        // nothing of the capture ran: issue plainly, and no graphs from now on
+        // the capture was lost (another thread of the program waited for the
+        // device, say) and nothing of it ran: issue plainly
         cudaGetLastError();
         if (exec) cudaGraphExecDestroy(exec);
-        g->graphs_off = true;
+        ++g->graphs_failed;
         c->launches = launches0;
         return issue();
     }
@@ -3345,6 +3350,13 @@ int vg_gkr_tables_rewind(vg_gkr *g)
     g->n = 0;
     g->round0_pending = false;
     return VG_OK;
+}
+
+void vg_gkr_tables_discard(vg_gkr *g)
+{
+    g->pend_launch.clear();
+    g->pend_r.clear();
+    g->held = g->gather_pending = g->round0_pending = false;
 }
 
 int vg_gkr_tables_begin(vg_gkr *g, const vg_fe *V, long n, vg_fe **AV, vg_fe **AM)

@@ -6,6 +6,11 @@
 #pragma once
 #include "virgo_b200.h"
 
+// A graph capture can be lost to another thread of the program (one that waits
+// for the whole device); its launches are then issued plainly.  An object that
+// lost this many captures for any reason makes no more graphs.
+constexpr int MAX_LOST_CAPTURES = 3;
+
 // ---- GKR (gkr.cu) ----
 // Deferred mode on: rounds and v_res write records of 9 values on the device
 // (round: the 3 sums, then the 6 folded values when one pair remained;
@@ -29,6 +34,8 @@ void vg_gkr_graph_counts(const vg_gkr *g, long long *replays, long long *capture
 int vg_gkr_tables_create(vg_ctx *ctx, long max_n, int max_records, vg_gkr **out);
 int vg_gkr_tables_reserve(vg_gkr *g, long max_n, int max_records);
 int vg_gkr_tables_rewind(vg_gkr *g);
+// Forgets the rounds still queued (their captured launches were lost).
+void vg_gkr_tables_discard(vg_gkr *g);
 int vg_gkr_tables_begin(vg_gkr *g, const vg_fe *V, long n, vg_fe **AV, vg_fe **AM);
 const vg_fe *vg_gkr_records_dev(const vg_gkr *g);
 int vg_gkr_record_count(const vg_gkr *g);
